@@ -12,9 +12,16 @@ template <class T, bool UP>
 cudaError_t trailing_update(T* A, long long lda, int k0, int nbk, int n, long long t0, int cols, const int* dinfo,
                             cudaStream_t st);
 
-// X * L11^H = A21 for the rows below the diagonal block [k0, k0+nbk) (potrf.cu).
-template <class T, bool UP>
-cudaError_t launch_trsm_panel(T* A, long long lda, int k0, int nbk, int n, const int* dinfo, cudaStream_t s);
+// The diagonal block [k0, k0+nbk)^2 (nbk <= 128) of each matrix of a batch (astride
+// elements and one info word apart), FP64 arithmetic for either storage (panel.cu).
+template <class S, bool UP>
+cudaError_t launch_potrf_diag(S* A, long long lda, long long astride, int batch, int k0, int nbk, int* dinfo,
+                              cudaStream_t st);
+
+// X * L11^T = A21 for the rows below that block (panel.cu).
+template <class S, bool UP>
+cudaError_t launch_trsm_panel_dmma(S* A, long long lda, long long astride, int batch, int k0, int nbk, int n,
+                                   const int* dinfo, cudaStream_t st);
 
 // The FP64 lower update of the region from row / column t0 (all of it, or its
 // first cols columns when cols > 0) over a batch of equal-order matrices

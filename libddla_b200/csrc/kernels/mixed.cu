@@ -2,9 +2,8 @@
 //
 // The FP64 matrix A (lower) is copied to an FP32 working matrix W; W is
 // factored with the blocked right-looking scheme of potrf.cu, but
-//   * each diagonal block is factored in FP64 (FP32 storage widened in shared
-//     memory, diag_factor.cuh) and rounded back to FP32;
-//   * the panel solve runs in FP32 on W (k_trsm_panel<float>);
+//   * each diagonal block is factored and its panel solved in FP64 arithmetic on the
+//     FP64 tensor cores (FP32 storage, panel.cu);
 //   * the panel is packed into a K-contiguous operand copy P (BF16, or FP32
 //     rounded to TF32) and the trailing update C -= P_I P_J^T runs on the
 //     5th-generation tensor cores: one elected thread issues tcgen05.mma into a
@@ -23,7 +22,6 @@
 
 #include "common.cuh"
 #include "ddla_kernels_internal.h"
-#include "diag_factor.cuh"
 #include "profile.h"
 #include "tc_common.cuh"
 
@@ -96,73 +94,6 @@ __global__ void __launch_bounds__(256) k_max_nonneg(const double* __restrict__ v
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) m = fmax(m, v[i]);
     for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_down_sync(0xffffffffu, m, o));
     if ((threadIdx.x & 31) == 0) atomicMax(reinterpret_cast<unsigned long long*>(out), __double_as_longlong(m));
-}
-
-// ---------------------------------------------------------------------------
-// diagonal block: FP32 storage, FP64 arithmetic
-// ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) k_potrf_diag_mixed(float* __restrict__ W, long long ldw, int k0, int nbk,
-                                                          int* __restrict__ info)
-{
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    double* s = reinterpret_cast<double*>(smem_raw);
-    const int ld = diag_block_ld<double>(nbk);
-    if (*(volatile int*)info != 0) return;
-    const int total = nbk * nbk;
-    const float* Wb = W + k0 + (long long)k0 * ldw;
-    if (nbk == 128) {
-        // the full block by float4 columns (ldw and k0 are multiples of 4): 32 per column,
-        // consecutive threads down a column; groups wholly above the diagonal are skipped
-#pragma unroll 4
-        for (int idx = threadIdx.x; idx < 128 * 32; idx += 256) {
-            const int q = idx & 31, j = idx >> 5;
-            if (4 * q + 3 < j) continue;
-            const float4 v = *reinterpret_cast<const float4*>(Wb + 4 * q + (long long)j * ldw);
-            double* d = s + 4 * q + j * ld;
-            d[0] = v.x;
-            d[1] = v.y;
-            d[2] = v.z;
-            d[3] = v.w;
-        }
-    } else {
-        for (int base = 0; base < total; base += 16 * 256) {
-            float v[16];
-#pragma unroll
-            for (int u = 0; u < 16; ++u) {
-                const int idx = base + u * 256 + threadIdx.x;
-                const int i = idx % nbk, j = idx / nbk;
-                v[u] = (idx < total && i >= j) ? Wb[i + (long long)j * ldw] : 0.f;
-            }
-#pragma unroll
-            for (int u = 0; u < 16; ++u) {
-                const int idx = base + u * 256 + threadIdx.x;
-                if (idx < total) s[(idx % nbk) + (idx / nbk) * ld] = (double)v[u];
-            }
-        }
-    }
-    __syncthreads();
-    const int fail = factor_block_smem<double>(s, ld, nbk);
-    if (nbk == 128) {
-        // float4 stores of the lower part; a group crossing the diagonal keeps its upper entries
-        for (int idx = threadIdx.x; idx < 128 * 32; idx += 256) {
-            const int q = idx & 31, j = idx >> 5;
-            if (4 * q + 3 < j) continue;
-            float* dst = W + k0 + 4 * q + (long long)(k0 + j) * ldw;
-            const double* src = s + 4 * q + j * ld;
-            if (4 * q >= j) {
-                *reinterpret_cast<float4*>(dst) = make_float4((float)src[0], (float)src[1], (float)src[2], (float)src[3]);
-            } else {
-                for (int e = 0; e < 4; ++e)
-                    if (4 * q + e >= j) dst[e] = (float)src[e];
-            }
-        }
-    } else {
-        for (int idx = threadIdx.x; idx < total; idx += blockDim.x) {
-            const int i = idx % nbk, j = idx / nbk;
-            if (i >= j) W[(k0 + i) + (long long)(k0 + j) * ldw] = (float)s[i + j * ld];
-        }
-    }
-    if (fail && threadIdx.x == 0) *info = k0 + fail;
 }
 
 // ---------------------------------------------------------------------------
@@ -1220,8 +1151,6 @@ cudaError_t potrf_mixed_enqueue(float* W, long long ldw, int n, int G, void* P0,
                                 cudaStream_t st)
 {
     constexpr int NB = MX_NB;
-    const size_t diag_smem = (size_t)NB * diag_block_ld<double>(NB) * sizeof(double);
-    if (cudaError_t e = smem_optin(k_potrf_diag_mixed, diag_smem); e != cudaSuccess) return e;
     MixedStreams& L = mixed_streams();
     cudaStream_t hi = L.hi;
     void* P[2] = {P0, P1};
@@ -1231,11 +1160,10 @@ cudaError_t potrf_mixed_enqueue(float* W, long long ldw, int n, int G, void* P0,
         const int nbk = n - k0 < NB ? n - k0 : NB;
         {
             ProfScope ps(PK_MIXED_OTHER, s, (double)nbk * nbk * nbk / 3.0, 4.0 * nbk * (nbk + 1));
-            k_potrf_diag_mixed<<<1, 256, (size_t)nbk * diag_block_ld<double>(nbk) * sizeof(double), s>>>(W, ldw, k0, nbk, dinfo);
+            if (cudaError_t de = launch_potrf_diag<float, false>(W, ldw, 0, 1, k0, nbk, dinfo, s); de != cudaSuccess)
+                return de;
         }
-        note_launches(1);
-        if ((long long)n - k0 - nbk <= 0) return cudaGetLastError();
-        return launch_trsm_panel<float, false>(W, ldw, k0, nbk, n, dinfo, s);
+        return launch_trsm_panel_dmma<float, false>(W, ldw, 0, 1, k0, nbk, n, dinfo, s);
     };
     // rows [pr0, n) x columns [k0, k0 + kw) of W -> K-contiguous operand at Pbuf
     auto pack = [&](long long pr0, int k0, int kw, void* Pbuf, cudaStream_t s) -> cudaError_t {
@@ -1329,8 +1257,6 @@ cudaError_t potrf_mixed_stream_enqueue(int n, int G, const double* Ah, long long
                                        double* anrm, int* dinfo, int* status, cudaStream_t cs, cudaStream_t st)
 {
     constexpr int NB = MX_NB;
-    const size_t diag_smem = (size_t)NB * diag_block_ld<double>(NB) * sizeof(double);
-    if (cudaError_t e = smem_optin(k_potrf_diag_mixed, diag_smem); e != cudaSuccess) return e;
     const long long SW = (long long)G * NB;
     const size_t esz = TF32 ? 4 : 2;
     const int S = (int)ceil_div(n, SW);
@@ -1407,12 +1333,11 @@ cudaError_t potrf_mixed_stream_enqueue(int n, int G, const double* Ah, long long
                 break;
             {
                 ProfScope ps(PK_MIXED_OTHER, hs, (double)nbk * nbk * nbk / 3.0, 4.0 * nbk * (nbk + 1));
-                k_potrf_diag_mixed<<<1, 256, (size_t)nbk * diag_block_ld<double>(nbk) * sizeof(double), hs>>>(W, ldw, (int)kg, nbk,
-                                                                                             dinfo);
+                e = launch_potrf_diag<float, false>(W, ldw, 0, 1, (int)kg, nbk, dinfo, hs);
             }
-            note_launches(1);
+            if (e != cudaSuccess) break;
             if (kg + nbk >= n) break;  // the last block column: nothing to its right
-            if ((e = launch_trsm_panel<float, false>(W, ldw, (int)kg, nbk, n, dinfo, hs)) != cudaSuccess) break;
+            if ((e = launch_trsm_panel_dmma<float, false>(W, ldw, 0, 1, (int)kg, nbk, n, dinfo, hs)) != cudaSuccess) break;
             {
                 const long long m = (long long)n - kg;
                 ProfScope ps(PK_MIXED_OTHER, hs, 0.0, (double)m * NB * (4.0 + (TF32 ? 4.0 : 2.0)));

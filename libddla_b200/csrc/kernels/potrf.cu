@@ -3,10 +3,12 @@
 //
 // Replaces the vendor call the reference makes at src/Cholesky/potrf.cpp:106-113
 // (cusolverDn?potrf).  Per block column k of width NB:
-//   1. k_potrf_diag   -- the NB x NB diagonal block in shared memory, factored in
-//                        32-wide steps (diag_factor.cuh); info detected in-kernel;
-//   2. k_trsm_panel   -- L21 = A21 * L11^{-H}: warps own rows, lanes own columns,
-//                        each solved entry broadcast with a warp shuffle;
+//   1. the NB x NB diagonal block: real types on the FP64 tensor cores
+//      (k_potrf_diag_dmma, panel.cu), complex types in shared memory in 32-wide
+//      steps (k_potrf_diag, diag_factor.cuh); info detected in-kernel;
+//   2. L21 = A21 * L11^{-H}: real types on the FP64 tensor cores
+//      (k_trsm_panel_dmma, panel.cu); complex types by k_trsm_panel, warps own
+//      rows, lanes own columns, each solved entry broadcast with a warp shuffle;
 //   3. trailing update -- C -= L21 * L21^H on lower tiles (FP64 DMMA for double,
 //                        syrk.cu; register-tiled SIMT for the other types).
 // Look-ahead: the update of block column k+1 plus the diagonal block and panel
@@ -33,14 +35,12 @@ namespace ddlak {
 // 1. diagonal block
 // ---------------------------------------------------------------------------
 template <class T, bool UP>
-__global__ void __launch_bounds__(256) k_potrf_diag(T* __restrict__ A, long long lda, long long astride, int k0,
-                                                    int nbk, int* __restrict__ info)
+__global__ void __launch_bounds__(256) k_potrf_diag(T* __restrict__ A, long long lda, int k0, int nbk,
+                                                    int* __restrict__ info)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     T* s = reinterpret_cast<T*>(smem_raw);
-    const int ld = diag_block_ld<T>(nbk);
-    A += (long long)blockIdx.x * astride;  // blockIdx.x: the matrix of a batch (grid 1 for one matrix)
-    info += blockIdx.x;
+    const int ld = diag_block_ld(nbk);
     if (*(volatile int*)info != 0) return;
     load_lview_block<T, UP>(s, ld, A, lda, k0, k0, nbk, nbk, nbk, nbk, true);
     const int fail = factor_block_smem<T>(s, ld, nbk);
@@ -244,329 +244,42 @@ DDLAK_INST_SIMT(cf64, true)
 // ---------------------------------------------------------------------------
 template <class T> constexpr int potrf_nb() { return sizeof(T) == 16 ? 64 : 128; }
 
-// ---------------------------------------------------------------------------
-// The FP32 panel of the mixed factorization (lower storage, nbk <= 128): one
-// thread per row.  X L11^T = A21 along the row, in two halves of 64 columns so
-// that at most 64 of the row's values are live in registers:
-//   1. x1 = row[0:64] solved against L11[0:64, 0:64] (x_j *= 1 / l_jj,
-//      x_k -= x_j l_kj for k > j), written back and staged in shared memory;
-//   2. x2 = row[64:128] - x1 L11[64:128, 0:64]^T, then solved against
-//      L11[64:128, 64:128], written back.
-// Columns of L11 are read from shared memory as float4 broadcasts (every thread
-// of the warp reads the same address); the row loads and stores are coalesced
-// (consecutive threads, consecutive rows of the column-major panel), and no
-// shuffle sits on the per-column chain.
-// ---------------------------------------------------------------------------
-constexpr int TRR_NT = 128;
-constexpr size_t TRR_SMEM = (128 * 128 + 64 * TRR_NT) * sizeof(float);
-
-// a shared-memory float4 load kept in program order (the unrolled substitution would
-// otherwise hoist hundreds of them ahead of their use and run out of registers)
-__device__ __forceinline__ float4 ld_shared_f4(const float4* p)
-{
-    float4 v;
-    const unsigned a = (unsigned)__cvta_generic_to_shared(p);
-    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a));
-    return v;
-}
-
-// x (64 values at column offset c0) against the 64 x 64 diagonal part of L11 at (c0, c0)
-__device__ __forceinline__ void trr_solve64(float (&x)[64], const float* l11, const float* rinv, int c0)
-{
-#pragma unroll
-    for (int j = 0; j < 64; ++j) {
-        x[j] *= rinv[c0 + j];
-        const float4* col = reinterpret_cast<const float4*>(&l11[(c0 + j) * 128 + c0]);
-#pragma unroll
-        for (int q = 0; q < 16; ++q) {
-            if (4 * q + 3 > j) {
-                const float4 l = ld_shared_f4(col + q);
-                if (4 * q + 0 > j) x[4 * q + 0] = fmaf(-x[j], l.x, x[4 * q + 0]);
-                if (4 * q + 1 > j) x[4 * q + 1] = fmaf(-x[j], l.y, x[4 * q + 1]);
-                if (4 * q + 2 > j) x[4 * q + 2] = fmaf(-x[j], l.z, x[4 * q + 2]);
-                if (4 * q + 3 > j) x[4 * q + 3] = fmaf(-x[j], l.w, x[4 * q + 3]);
-            }
-        }
-    }
-}
-
-__device__ int g_trsm_status;  // a TMA wait that gave up (never expected): the panel is NaN-poisoned
-
-// TMA: L11 staged by one 128 x 128 TMA box (nbk = 128; the solve reads only entries
-// below the diagonal, so the block's upper half comes in unmasked); otherwise by loads.
-template <bool TMA>
-__global__ void __launch_bounds__(TRR_NT) k_trsm_panel_rows(const __grid_constant__ CUtensorMap amap,
-                                                            float* __restrict__ A, long long lda, int k0, int nbk,
-                                                            int n, const int* __restrict__ info)
-{
-    extern __shared__ __align__(128) float trr_smem[];
-    float* l11 = trr_smem;               // l11[j * 128 + k] = L(k0 + k, k0 + j) (zero for k < j or k >= nbk by loads)
-    float* xs = trr_smem + 128 * 128;    // xs[j * TRR_NT + t]: thread t's solved first half
-    __shared__ float rinv[128];
-    __shared__ __align__(8) uint64_t l11_bar;
-    if (*(volatile const int*)info != 0) return;
-    bool staged = true;
-    if constexpr (TMA) {
-        if (threadIdx.x == 0) {
-            tc::mbar_init(&l11_bar, 1);
-            tc::mbar_fence_init();
-            tc::prefetch_tmap(&amap);
-            tc::mbar_expect_tx(&l11_bar, 128 * 128 * 4);
-            tc::tma_load_2d(l11, &amap, &l11_bar, k0, k0);
-        }
-        __syncthreads();
-        staged = __syncthreads_and(tc::mbar_wait(&l11_bar, 0, &g_trsm_status, 0x53));
-        if (!staged && threadIdx.x == 0) (void)tc::mbar_wait(&l11_bar, 0, &g_trsm_status, 0x54);
-    } else {
-        const float* Ad = A + k0 + (long long)k0 * lda;
-        for (int idx = threadIdx.x; idx < 128 * 32; idx += TRR_NT) {
-            const int j = idx >> 5, k4 = (idx & 31) * 4;
-            float v[4];
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const int k = k4 + e;
-                v[e] = (j < nbk && k < nbk && k >= j) ? Ad[k + (long long)j * lda] : 0.f;
-            }
-            *reinterpret_cast<float4*>(&l11[j * 128 + k4]) = make_float4(v[0], v[1], v[2], v[3]);
-        }
-        __syncthreads();
-    }
-    rinv[threadIdx.x] = threadIdx.x < nbk ? 1.f / l11[threadIdx.x * 129] : 0.f;
-    __syncthreads();
-    const int t = threadIdx.x;
-    const long long row = (long long)k0 + nbk + (long long)blockIdx.x * TRR_NT + t;
-    const bool live = row < n;
-    float* Ar = A + (live ? row : (long long)k0) + (long long)k0 * lda;
-    if (!staged) {  // L11 never arrived: poison the rows (the next diagonal block reports a NaN pivot)
-        if (live)
-            for (int c = 0; c < nbk; ++c) Ar[(long long)c * lda] = __int_as_float(0x7fc00000);
-        return;
-    }
-    // the two 64-column halves through one rolled loop, so that the unrolled solve exists once
-    // in the instruction stream (the kernel is bound by instruction fetch, not arithmetic)
-#pragma unroll 1
-    for (int half = 0; half < 2; ++half) {
-        const int c0 = 64 * half;
-        if (c0 >= nbk) break;  // uniform
-        float x[64];
-        {
-            const float* p = Ar + (long long)c0 * lda;
-#pragma unroll
-            for (int c = 0; c < 64; ++c) x[c] = (live && c0 + c < nbk) ? p[(long long)c * lda] : 0.f;
-        }
-        if (half == 1) {
-            // x -= x1 L11[64:128, 0:64]^T, x1 = this thread's solved first half
-#pragma unroll 4
-            for (int j = 0; j < 64; ++j) {
-                const float xj = xs[j * TRR_NT + t];
-                const float4* col = reinterpret_cast<const float4*>(&l11[j * 128 + 64]);
-#pragma unroll
-                for (int q = 0; q < 16; ++q) {
-                    const float4 l = ld_shared_f4(col + q);
-                    x[4 * q + 0] = fmaf(-xj, l.x, x[4 * q + 0]);
-                    x[4 * q + 1] = fmaf(-xj, l.y, x[4 * q + 1]);
-                    x[4 * q + 2] = fmaf(-xj, l.z, x[4 * q + 2]);
-                    x[4 * q + 3] = fmaf(-xj, l.w, x[4 * q + 3]);
-                }
-            }
-        }
-        trr_solve64(x, l11, rinv, c0);
-        {
-            // the row's addresses are recomputed here rather than kept live through the solve
-            float* p = Ar + (long long)c0 * lda;
-            long long ld = lda;
-            asm volatile("" : "+l"(p), "+l"(ld));
-#pragma unroll
-            for (int c = 0; c < 64; ++c) {
-                if (live && c0 + c < nbk) p[(long long)c * ld] = x[c];
-                if (half == 0) xs[c * TRR_NT + t] = x[c];
-            }
-        }
-    }
-}
-
-// ---------------------------------------------------------------------------
-// The FP64 panel (lower storage, nbk <= 128): L11 staged in shared memory by TMA
-// (ten 32 x 32 boxes, one mbarrier) when lda is even, then one thread per row, in
-// four chunks of 32 columns so that 32 of the row's values are live in registers.
-// Chunk C: x = row[32C : 32C + 32]; x -= x_J L11[32C.., 32J..]^T for the
-// chunks J < C (their solved values re-read from the row this thread already
-// wrote); then x is solved against the diagonal block (x_j *= 1 / l_jj,
-// x_k -= x_j l_kj for k > j) and written back.  Every entry receives the
-// updates of its columns in increasing order, as in the column-by-column
-// substitution.  L11's lower part is held as ten 32 x 32 blocks (80 KB, two
-// CTAs per SM) read as 16-byte broadcasts; the row loads and stores are
-// coalesced (consecutive threads, consecutive rows).
-// ---------------------------------------------------------------------------
-constexpr int TRD_NT = 128;
-constexpr size_t TRD_SMEM = 10 * 32 * 32 * sizeof(double);
-
-__device__ __forceinline__ double2 ld_shared_d2(const double2* p)
-{
-    double2 v;
-    const unsigned a = (unsigned)__cvta_generic_to_shared(p);
-    asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "r"(a));
-    return v;
-}
-
-// TMA_DIMS: 0 = L11 staged by plain loads (any lda, any nbk); 2 = by ten 32 x 32 TMA
-// boxes from a 2-D map over A; 3 = the same from a 3-D map over a batch (z = matrix).
-// The TMA forms need nbk = 128: they load whole boxes, so the diagonal blocks'
-// upper halves come in unmasked (the solve reads only entries below the diagonal).
-
-template <int TMA_DIMS>
-__global__ void __launch_bounds__(TRD_NT) k_trsm_panel_rows_f64(const __grid_constant__ CUtensorMap amap,
-                                                                double* __restrict__ A, long long lda,
-                                                                long long astride, int k0, int nbk, int n,
-                                                                const int* __restrict__ info)
-{
-    // block (C, J), J <= C, at trd_smem + (C (C + 1) / 2 + J) * 1024, element [j * 32 + i]
-    // = L(k0 + 32 C + i, k0 + 32 J + j) (zero above the diagonal and past nbk when staged by loads)
-    extern __shared__ __align__(128) double trd_smem[];
-    __shared__ double rinv[128];
-    __shared__ __align__(8) uint64_t l11_bar;
-    A += (long long)blockIdx.y * astride;  // blockIdx.y: the matrix of a batch
-    info += blockIdx.y;
-    if (*(volatile const int*)info != 0) return;
-    bool staged = true;
-    if constexpr (TMA_DIMS == 0) {
-        const double* Ad = A + k0 + (long long)k0 * lda;
-        for (int idx = threadIdx.x; idx < 10 * 1024; idx += TRD_NT) {
-            const int b = idx >> 10, e = idx & 1023, j = e >> 5, i = e & 31;
-            const int C = b >= 6 ? 3 : b >= 3 ? 2 : b >= 1 ? 1 : 0;
-            const int J = b - C * (C + 1) / 2;
-            const int r = 32 * C + i, c = 32 * J + j;
-            trd_smem[idx] = (r < nbk && c < nbk && r >= c) ? Ad[r + (long long)c * lda] : 0.0;
-        }
-        __syncthreads();
-    } else {
-        if (threadIdx.x == 0) {
-            tc::mbar_init(&l11_bar, 1);
-            tc::mbar_fence_init();
-            tc::prefetch_tmap(&amap);
-            tc::mbar_expect_tx(&l11_bar, 10 * 32 * 32 * 8);
-            for (int C = 0, b = 0; C < 4; ++C)
-                for (int J = 0; J <= C; ++J, ++b) {
-                    if constexpr (TMA_DIMS == 2)
-                        tc::tma_load_2d(trd_smem + b * 1024, &amap, &l11_bar, k0 + 32 * C, k0 + 32 * J);
-                    else
-                        tc::tma_load_3d(trd_smem + b * 1024, &amap, &l11_bar, k0 + 32 * C, k0 + 32 * J,
-                                        (int)blockIdx.y);
-                }
-        }
-        __syncthreads();
-        staged = __syncthreads_and(tc::mbar_wait(&l11_bar, 0, &g_trsm_status, 0x51));
-        if (!staged && threadIdx.x == 0)  // give the copies a second bounded chance to land before the exit
-            (void)tc::mbar_wait(&l11_bar, 0, &g_trsm_status, 0x52);
-    }
-    {
-        const int t = threadIdx.x, C = t >> 5, i = t & 31;
-        rinv[t] = t < nbk ? 1.0 / trd_smem[(C * (C + 1) / 2 + C) * 1024 + i * 32 + i] : 0.0;
-    }
-    __syncthreads();
-    const long long row = (long long)k0 + nbk + (long long)blockIdx.x * TRD_NT + threadIdx.x;
-    const bool live = row < n;
-    double* Ar = A + (live ? row : (long long)k0) + (long long)k0 * lda;
-    if (!staged) {  // L11 never arrived: poison the rows (the next diagonal block reports a NaN pivot)
-        if (live)
-            for (int c = 0; c < nbk; ++c) Ar[(long long)c * lda] = __longlong_as_double(0x7ff8000000000000LL);
-        return;
-    }
-    const int nch = (nbk + 31) >> 5;
-    for (int C = 0; C < nch; ++C) {
-        double x[32];
-#pragma unroll
-        for (int i = 0; i < 32; ++i) x[i] = (live && 32 * C + i < nbk) ? Ar[(long long)(32 * C + i) * lda] : 0.0;
-        for (int J = 0; J < C; ++J) {
-            const double* blk = trd_smem + (C * (C + 1) / 2 + J) * 1024;
-            const double* xs = Ar + (long long)(32 * J) * lda;
-#pragma unroll 4
-            for (int j = 0; j < 32; ++j) {
-                const double xj = live ? xs[(long long)j * lda] : 0.0;
-                const double2* col = reinterpret_cast<const double2*>(blk + j * 32);
-#pragma unroll
-                for (int h = 0; h < 16; ++h) {
-                    const double2 l = ld_shared_d2(col + h);
-                    x[2 * h] = fma(-xj, l.x, x[2 * h]);
-                    x[2 * h + 1] = fma(-xj, l.y, x[2 * h + 1]);
-                }
-            }
-        }
-        const double* dblk = trd_smem + (C * (C + 1) / 2 + C) * 1024;
-#pragma unroll
-        for (int j = 0; j < 32; ++j) {
-            x[j] *= rinv[32 * C + j];
-            const double2* col = reinterpret_cast<const double2*>(dblk + j * 32);
-#pragma unroll
-            for (int h = 0; h < 16; ++h) {
-                if (2 * h + 1 > j) {
-                    const double2 l = ld_shared_d2(col + h);
-                    if (2 * h > j) x[2 * h] = fma(-x[j], l.x, x[2 * h]);
-                    x[2 * h + 1] = fma(-x[j], l.y, x[2 * h + 1]);
-                }
-            }
-        }
-#pragma unroll
-        for (int i = 0; i < 32; ++i)
-            if (live && 32 * C + i < nbk) Ar[(long long)(32 * C + i) * lda] = x[i];
-    }
-}
-
+// The diagonal block: real types on the FP64 tensor cores (panel.cu), complex types
+// in shared memory.
 template <class T, bool UP>
-cudaError_t launch_trsm_panel(T* A, long long lda, int k0, int nbk, int n, const int* dinfo, cudaStream_t s)
+static cudaError_t diag_block(T* A, long long lda, int k0, int nbk, int* dinfo, cudaStream_t s)
 {
-    if constexpr (std::is_same<T, float>::value && !UP) {
-        const long long m = (long long)n - k0 - nbk;
-        if (m <= 0) return cudaSuccess;
-        const double md = (double)m, b = nbk;
-        ProfScope ps(PK_TRSM_PANEL, s, md * b * b, sizeof(T) * (2.0 * md * b + b * (b + 1) / 2));
-        const unsigned grid = (unsigned)ceil_div(m, TRR_NT);
-        CUtensorMap amap{};
-        if (nbk == 128 && (lda % 4) == 0 &&
-            tc::encode_colmajor_2d(&amap, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, A, n, n, lda, 128, 128,
-                                   CU_TENSOR_MAP_SWIZZLE_NONE)) {
-            if (cudaError_t e = smem_optin(k_trsm_panel_rows<true>, TRR_SMEM); e != cudaSuccess) return e;
-            k_trsm_panel_rows<true><<<grid, TRR_NT, TRR_SMEM, s>>>(amap, A, lda, k0, nbk, n, dinfo);
-        } else {
-            if (cudaError_t e = smem_optin(k_trsm_panel_rows<false>, TRR_SMEM); e != cudaSuccess) return e;
-            k_trsm_panel_rows<false><<<grid, TRR_NT, TRR_SMEM, s>>>(amap, A, lda, k0, nbk, n, dinfo);
-        }
+    const double cf = Traits<T>::cplx ? 4.0 : 1.0, b = nbk;
+    ProfScope ps(PK_POTRF_DIAG, s, cf * b * b * b / 3.0, sizeof(T) * b * (b + 1));
+    if constexpr (!Traits<T>::cplx) {
+        return launch_potrf_diag<T, UP>(A, lda, 0, 1, k0, nbk, dinfo, s);
+    } else {
+        k_potrf_diag<T, UP><<<1, 256, (size_t)nbk * diag_block_ld(nbk) * sizeof(T), s>>>(A, lda, k0, nbk, dinfo);
         note_launches(1);
         return cudaGetLastError();
     }
-    if constexpr (std::is_same<T, double>::value && !UP) {
-        const long long m = (long long)n - k0 - nbk;
-        if (m <= 0) return cudaSuccess;
-        const double md = (double)m, b = nbk;
-        ProfScope ps(PK_TRSM_PANEL, s, md * b * b, sizeof(T) * (2.0 * md * b + b * (b + 1) / 2));
-        const unsigned grid = (unsigned)ceil_div(m, TRD_NT);
-        CUtensorMap amap{};
-        if (nbk == 128 && !(lda & 1) &&
-            tc::encode_colmajor_2d(&amap, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 8, A, n, n, lda, 32, 32,
-                                   CU_TENSOR_MAP_SWIZZLE_NONE)) {
-            if (cudaError_t e = smem_optin(k_trsm_panel_rows_f64<2>, TRD_SMEM); e != cudaSuccess) return e;
-            k_trsm_panel_rows_f64<2><<<grid, TRD_NT, TRD_SMEM, s>>>(amap, A, lda, 0, k0, nbk, n, dinfo);
-        } else {
-            if (cudaError_t e = smem_optin(k_trsm_panel_rows_f64<0>, TRD_SMEM); e != cudaSuccess) return e;
-            k_trsm_panel_rows_f64<0><<<grid, TRD_NT, TRD_SMEM, s>>>(amap, A, lda, 0, k0, nbk, n, dinfo);
-        }
-        note_launches(1);
-        return cudaGetLastError();
-    }
-    constexpr int NQ = potrf_nb<T>() / 32;
-    constexpr int PR = sizeof(T) >= 16 ? 4 : 8;
-    const size_t panel_smem = (size_t)(NQ * 32) * (NQ * 32 + 1) * sizeof(T);
-    const long long m = (long long)n - k0 - nbk;
-    if (m <= 0) return cudaSuccess;
-    if (cudaError_t e = smem_optin(k_trsm_panel<T, UP, NQ, PR>, panel_smem); e != cudaSuccess) return e;
-    const double cf = Traits<T>::cplx ? 4.0 : 1.0, md = (double)m, b = nbk;
-    ProfScope ps(PK_TRSM_PANEL, s, cf * md * b * b, sizeof(T) * (2.0 * md * b + b * (b + 1) / 2));
-    const long long grid = trsm_grid(k_trsm_panel<T, UP, NQ, PR>, panel_smem, ceil_div(m, 8 * PR));
-    k_trsm_panel<T, UP, NQ, PR><<<(unsigned)grid, 256, panel_smem, s>>>(A, lda, k0, nbk, n, dinfo);
-    note_launches(1);
-    return cudaGetLastError();
 }
-template cudaError_t launch_trsm_panel<float, false>(float*, long long, int, int, int, const int*, cudaStream_t);
+
+// X L11^H = A21 for the rows below it
+template <class T, bool UP>
+static cudaError_t panel_solve(T* A, long long lda, int k0, int nbk, int n, const int* dinfo, cudaStream_t s)
+{
+    if constexpr (!Traits<T>::cplx) {
+        return launch_trsm_panel_dmma<T, UP>(A, lda, 0, 1, k0, nbk, n, dinfo, s);
+    } else {
+        constexpr int NQ = potrf_nb<T>() / 32;
+        constexpr int PR = sizeof(T) >= 16 ? 4 : 8;
+        const size_t panel_smem = (size_t)(NQ * 32) * (NQ * 32 + 1) * sizeof(T);
+        const long long m = (long long)n - k0 - nbk;
+        if (m <= 0) return cudaSuccess;
+        const double md = (double)m, b = nbk;
+        ProfScope ps(PK_TRSM_PANEL, s, 4.0 * md * b * b, sizeof(T) * (2.0 * md * b + b * (b + 1) / 2));
+        const long long grid = trsm_grid(k_trsm_panel<T, UP, NQ, PR>, panel_smem, ceil_div(m, 8 * PR));
+        k_trsm_panel<T, UP, NQ, PR><<<(unsigned)grid, 256, panel_smem, s>>>(A, lda, k0, nbk, n, dinfo);
+        note_launches(1);
+        return cudaGetLastError();
+    }
+}
 
 namespace {
 struct LookaheadRes {
@@ -595,12 +308,14 @@ template <class T, bool UP>
 static cudaError_t potrf_enqueue(T* A, long long lda, int n, int G, int* dinfo, cudaStream_t st)
 {
     constexpr int NB = potrf_nb<T>();
-    constexpr int NQ = NB / 32;
-    constexpr int PR = sizeof(T) >= 16 ? 4 : 8;
-    const size_t diag_smem = (size_t)NB * diag_block_ld<T>(NB) * sizeof(T);
-    const size_t panel_smem = (size_t)(NQ * 32) * (NQ * 32 + 1) * sizeof(T);
-    if (cudaError_t e = smem_optin(k_potrf_diag<T, UP>, diag_smem); e != cudaSuccess) return e;
-    if (cudaError_t e = smem_optin(k_trsm_panel<T, UP, NQ, PR>, panel_smem); e != cudaSuccess) return e;
+    if constexpr (Traits<T>::cplx) {
+        constexpr int NQ = NB / 32;
+        constexpr int PR = sizeof(T) >= 16 ? 4 : 8;
+        const size_t diag_smem = (size_t)NB * diag_block_ld(NB) * sizeof(T);
+        const size_t panel_smem = (size_t)(NQ * 32) * (NQ * 32 + 1) * sizeof(T);
+        if (cudaError_t e = smem_optin(k_potrf_diag<T, UP>, diag_smem); e != cudaSuccess) return e;
+        if (cudaError_t e = smem_optin(k_trsm_panel<T, UP, NQ, PR>, panel_smem); e != cudaSuccess) return e;
+    }
     const double cf = Traits<T>::cplx ? 4.0 : 1.0;  // real flops per multiply-add relative to a real one
     LookaheadRes& L = lookahead_res();
     cudaStream_t hi = L.hi;
@@ -608,27 +323,9 @@ static cudaError_t potrf_enqueue(T* A, long long lda, int n, int G, int* dinfo, 
     cudaError_t panel_err = cudaSuccess;
     auto diag_and_panel = [&](int k0, cudaStream_t s) {
         const int nbk = n - k0 < NB ? n - k0 : NB;
-        const double b = nbk;
-        {
-            ProfScope ps(PK_POTRF_DIAG, s, cf * b * b * b / 3.0, sizeof(T) * b * (b + 1));
-            k_potrf_diag<T, UP><<<1, 256, (size_t)nbk * diag_block_ld<T>(nbk) * sizeof(T), s>>>(A, lda, 0, k0, nbk,
-                                                                                              dinfo);
-        }
-        note_launches(1);
-        const long long m = (long long)n - k0 - nbk;
-        if (m <= 0) return;
-        if constexpr ((std::is_same<T, double>::value || std::is_same<T, float>::value) && !UP) {
-            const cudaError_t pe = launch_trsm_panel<T, UP>(A, lda, k0, nbk, n, dinfo, s);  // one thread per row
-            if (pe != cudaSuccess && panel_err == cudaSuccess) panel_err = pe;
-            return;
-        }
-        const double md = (double)m;
-        {
-            ProfScope ps(PK_TRSM_PANEL, s, cf * md * b * b, sizeof(T) * (2.0 * md * b + b * (b + 1) / 2));
-            const long long grid = trsm_grid(k_trsm_panel<T, UP, NQ, PR>, panel_smem, ceil_div(m, 8 * PR));
-            k_trsm_panel<T, UP, NQ, PR><<<(unsigned)grid, 256, panel_smem, s>>>(A, lda, k0, nbk, n, dinfo);
-        }
-        note_launches(1);
+        cudaError_t pe = diag_block<T, UP>(A, lda, k0, nbk, dinfo, s);
+        if (pe == cudaSuccess) pe = panel_solve<T, UP>(A, lda, k0, nbk, n, dinfo, s);
+        if (pe != cudaSuccess && panel_err == cudaSuccess) panel_err = pe;
     };
     // C -= L(:, k0 : k0 + kw) L(:, k0 : k0 + kw)^H on the region from row / column t0
     auto update = [&](int k0, int kw, long long t0, int cols, cudaStream_t s) -> cudaError_t {
@@ -817,36 +514,17 @@ extern "C" int ddlak_potrf_batched_f64(int batch, int n, void* A_, long long lda
     cudaError_t e = cudaMemsetAsync(dinfo, 0, sizeof(int) * (size_t)batch, st);
     if (e != cudaSuccess || n == 0) return (int)e;
     constexpr int NB = 128, G = BATCHED_POTRF_GROUP;
-    const size_t diag_smem = (size_t)NB * diag_block_ld<double>(NB) * sizeof(double);
-    if ((e = smem_optin(k_potrf_diag<double, false>, diag_smem)) != cudaSuccess) return (int)e;
-    if ((e = smem_optin(k_trsm_panel_rows_f64<3>, TRD_SMEM)) != cudaSuccess) return (int)e;
-    if ((e = smem_optin(k_trsm_panel_rows_f64<0>, TRD_SMEM)) != cudaSuccess) return (int)e;
-    // L11 of every matrix by TMA boxes of 32 x 32 (lda and astride even, A 16-byte aligned: checked above)
-    CUtensorMap amap{};
-    const bool tma = tc::encode_colmajor_3d(&amap, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 8, A, n, n, lda, batch, astride,
-                                            32, 32);
     const double nb3 = (double)batch;
     auto diag_and_panel = [&](int k0) -> cudaError_t {
         const int nbk = n - k0 < NB ? n - k0 : NB;
         const double b = nbk;
         {
             ProfScope ps(PK_POTRF_DIAG, st, nb3 * b * b * b / 3.0, nb3 * 8.0 * b * (b + 1));
-            k_potrf_diag<double, false><<<(unsigned)batch, 256, (size_t)nbk * diag_block_ld<double>(nbk) * 8, st>>>(
-                A, lda, astride, k0, nbk, dinfo);
+            if (cudaError_t de = launch_potrf_diag<double, false>(A, lda, astride, batch, k0, nbk, dinfo, st);
+                de != cudaSuccess)
+                return de;
         }
-        note_launches(1);
-        const long long m = (long long)n - k0 - nbk;
-        if (m > 0) {
-            const double md = (double)m;
-            ProfScope ps(PK_TRSM_PANEL, st, nb3 * md * b * b, nb3 * 8.0 * (2.0 * md * b + b * (b + 1) / 2));
-            const dim3 grid((unsigned)ceil_div(m, TRD_NT), (unsigned)batch);
-            if (tma && nbk == 128)
-                k_trsm_panel_rows_f64<3><<<grid, TRD_NT, TRD_SMEM, st>>>(amap, A, lda, astride, k0, nbk, n, dinfo);
-            else
-                k_trsm_panel_rows_f64<0><<<grid, TRD_NT, TRD_SMEM, st>>>(amap, A, lda, astride, k0, nbk, n, dinfo);
-            note_launches(1);
-        }
-        return cudaGetLastError();
+        return launch_trsm_panel_dmma<double, false>(A, lda, astride, batch, k0, nbk, n, dinfo, st);
     };
     // C -= L(:, k0 : k0 + kw) L(:, k0 : k0 + kw)^T on the region from t0 (all of it, or cols columns)
     auto update = [&](int k0, int kw, long long t0, int cols) -> cudaError_t {
