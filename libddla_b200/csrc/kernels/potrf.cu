@@ -382,6 +382,17 @@ static cudaError_t potrf_enqueue(T* A, long long lda, int n, int G, int* dinfo, 
     return cudaGetLastError();
 }
 
+// Block columns per super-step.  A wide super-step reads and writes the trailing matrix
+// less often, but its left-looking updates (K up to 128 (G - 1) on one block column)
+// lie on the chain, which is all of the time at small orders.  FP64, ms with G = 1 / 2 /
+// 4 / 8: n = 2048 0.86 / 0.91 / 1.0 / 1.1; 5003 3.70 / 3.60 / 3.77 / 3.9; 8192 - / 8.99 /
+// 8.59 / 8.8; 16384 - / - / 52.4 / 50.1.
+static int potrf_group(char type, int n)
+{
+    if (type != 'd') return DDLAK_POTRF_GROUP;
+    return n < 3072 ? 1 : n < 6144 ? 2 : n < 12288 ? 4 : DDLAK_POTRF_GROUP;
+}
+
 template <class T>
 static cudaError_t potrf_typed(char uplo, int n, int G, void* A, long long lda, int* dinfo, cudaStream_t st)
 {
@@ -532,9 +543,7 @@ extern "C" int ddlak_potrf_batched_f64(int batch, int n, void* A_, long long lda
         const double cw = cols ? (double)cols : md;
         const double fl = cols ? 2.0 * b * (md * cw - cw * (cw - 1) / 2) : md * (md + 1) * b;
         ProfScope ps(PK_SYRK_UPDATE, st, nb3 * fl, nb3 * 8.0 * ((cols ? 2.0 * md * cw : md * (md + 1)) + md * b));
-        cudaError_t ue = cudaSuccess;
-        if (!launch_dmma_tma_batched(A, lda, astride, batch, k0, kw, n, t0, cols, dinfo, st, &ue))
-            return cudaErrorInvalidValue;
+        const cudaError_t ue = launch_syrk_batched(A, lda, astride, batch, k0, kw, n, t0, cols, dinfo, st);
         note_launches(1);
         return ue;
     };
@@ -594,5 +603,5 @@ extern "C" int ddlak_potrf_grouped(char type, char uplo, int group, int n, void*
 
 extern "C" int ddlak_potrf(char type, char uplo, int n, void* A, long long lda, int* dinfo, void* stream)
 {
-    return ddlak_potrf_grouped(type, uplo, DDLAK_POTRF_GROUP, n, A, lda, dinfo, stream);
+    return ddlak_potrf_grouped(type, uplo, ddlak::potrf_group(type, n), n, A, lda, dinfo, stream);
 }

@@ -3,13 +3,11 @@
 // This is the work the reference hands to cuSOLVER inside ?potrf
 // (src/Cholesky/potrf.cpp:111) and, on multi-rank grids, to herk/gemm
 // (src/Cholesky/ppotrf.cpp:212-238).  For double it runs on the FP64 tensor
-// cores: mma.sync m16n8k4 f64 (DMMA).  Each CTA owns one 128x128 lower tile of
-// the region, streams the two 128 x nbk panel slices through a 3-stage ring in
-// k chunks (cp.async, or TMA boxes), and keeps its accumulators in registers
-// (8 warps, each a 64x32 sub-tile = 4x4 DMMA fragments of 16x8).  Diagonal tiles
-// store only i >= j.  Complex double runs as two real DMMA products per
-// fragment; float and complex float use the SIMT kernel in potrf.cu.
+// cores: mma.sync m16n8k4 f64 (DMMA).  Complex double (lower) runs as two real
+// DMMA products per fragment; the other types use the SIMT kernel in potrf.cu.
 #include <cuda.h>
+
+#include <type_traits>
 
 #include "common.cuh"
 #include "ddla_kernels_internal.h"
@@ -20,22 +18,16 @@ namespace ddlak {
 
 namespace {
 
-constexpr int DM_BM = 128, DM_BK = 16, DM_LDS = DM_BM + 4;  // 132: conflict-free 8-byte fragment reads
-constexpr int DM_STAGE = 2 * DM_BK * DM_LDS;                 // doubles per stage (A and B slices)
-constexpr int DM_NSTAGE = 3;
-
-__device__ __forceinline__ void cp_async8(void* smem, const void* gmem, int bytes)
-{
-    const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(s), "l"(gmem), "r"(bytes) : "memory");
-}
 __device__ __forceinline__ void cp_async16(void* smem, const void* gmem, int bytes)
 {
     const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(s), "l"(gmem), "r"(bytes) : "memory");
 }
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+// one arrival on the mbarrier once the cp.async copies this thread has issued so far have landed
+__device__ __forceinline__ void cp_async_arrive(uint64_t* bar)
+{
+    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(tc::smem_u32(bar)) : "memory");
+}
 
 // D += A B over k = 4 on the FP64 tensor cores, for two 8-row blocks at once
 // (mma.sync m16n8k4 f64): lane (g = lane / 4, q = lane % 4) supplies A(g, q) and
@@ -49,352 +41,302 @@ __device__ __forceinline__ void dmma2(double (&u)[2], double (&v)[2], double a_u
                  : "d"(a_up), "d"(a_lo), "d"(b));
 }
 
-// One k chunk (16 columns of the panel) of the A rows [ri, ri+128) and the B
-// rows [rj, rj+128) into a stage: As[k][i], Bs[k][i].  Rows at or past their
-// limit and columns past nbk are zero-filled.  VEC2: two consecutive rows per
-// 16-byte copy (lower storage with even lda and a 16-byte aligned base).
-template <bool UP, bool VEC2>
-__device__ __forceinline__ void load_chunk(double* st, const double* __restrict__ A, long long lda, long long ri,
-                                           long long rj, long long alim, long long blim, int kcol0, int kc, int nbk)
-{
-    double* As = st;
-    double* Bs = st + DM_BK * DM_LDS;
-    if (VEC2) {
-        for (int idx = threadIdx.x; idx < (DM_BM / 2) * DM_BK; idx += blockDim.x) {
-            const int i = 2 * (idx % (DM_BM / 2)), k = idx / (DM_BM / 2);
-            const bool kin = kc + k < nbk;
-            const long long col = (long long)kcol0 + kc + k;
-            {
-                const long long r = ri + i;
-                const int bytes = (kin && r < alim) ? (r + 1 < alim ? 16 : 8) : 0;
-                cp_async16(&As[k * DM_LDS + i], bytes ? A + r + col * lda : A, bytes);
-            }
-            {
-                const long long r = rj + i;
-                const int bytes = (kin && r < blim) ? (r + 1 < blim ? 16 : 8) : 0;
-                cp_async16(&Bs[k * DM_LDS + i], bytes ? A + r + col * lda : A, bytes);
-            }
-        }
-    } else {
-        for (int idx = threadIdx.x; idx < DM_BM * DM_BK; idx += blockDim.x) {
-            int i, k;
-            if (UP) { k = idx % DM_BK; i = idx / DM_BK; } else { i = idx % DM_BM; k = idx / DM_BM; }
-            const bool kin = kc + k < nbk;
-            const long long col = (long long)kcol0 + kc + k;
-            {
-                const long long r = ri + i;
-                const bool v = kin && r < alim;
-                cp_async8(&As[k * DM_LDS + i], v ? (UP ? A + col + r * lda : A + r + col * lda) : A, v ? 8 : 0);
-            }
-            {
-                const long long r = rj + i;
-                const bool v = kin && r < blim;
-                cp_async8(&Bs[k * DM_LDS + i], v ? (UP ? A + col + r * lda : A + r + col * lda) : A, v ? 8 : 0);
-            }
-        }
-    }
-}
-
-template <bool UP, bool VEC2>
-__global__ void __launch_bounds__(256, 1) k_syrk_dmma(double* __restrict__ A, long long lda, int k0, int nbk, int n,
-                                                      long long t0, int cols, const int* __restrict__ info)
-{
-    extern __shared__ __align__(16) double sm[];
-    if (*(volatile const int*)info != 0) return;
-    int I, J;
-    if (cols == 0) {
-        tile_of_tri(blockIdx.x, I, J);
-    } else {
-        const int nct = (cols + DM_BM - 1) / DM_BM;
-        J = blockIdx.x % nct;
-        I = blockIdx.x / nct;
-        if (I < J) return;
-    }
-    const long long cend = cols == 0 ? (long long)n : t0 + cols;
-    const long long ri = t0 + (long long)I * DM_BM, rj = t0 + (long long)J * DM_BM;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int wm = warp >> 2, wn = warp & 3;  // 2 x 4 warps, 64 x 32 each
-    const int g = lane >> 2, q = lane & 3;
-
-    double acc[8][4][2];
-#pragma unroll
-    for (int a = 0; a < 8; ++a)
-#pragma unroll
-        for (int b = 0; b < 4; ++b) acc[a][b][0] = acc[a][b][1] = 0.0;
-
-    const int nchunks = (nbk + DM_BK - 1) / DM_BK;
-#pragma unroll
-    for (int s = 0; s < DM_NSTAGE - 1; ++s) {
-        if (s < nchunks) load_chunk<UP, VEC2>(sm + s * DM_STAGE, A, lda, ri, rj, n, cend, k0, s * DM_BK, nbk);
-        cp_async_commit();
-    }
-    for (int c = 0; c < nchunks; ++c) {
-        const int pre = c + DM_NSTAGE - 1;
-        if (pre < nchunks)
-            load_chunk<UP, VEC2>(sm + (pre % DM_NSTAGE) * DM_STAGE, A, lda, ri, rj, n, cend, k0, pre * DM_BK, nbk);
-        cp_async_commit();
-        cp_async_wait<DM_NSTAGE - 1>();
-        __syncthreads();
-        const double* As = sm + (c % DM_NSTAGE) * DM_STAGE;
-        const double* Bs = As + DM_BK * DM_LDS;
-#pragma unroll
-        for (int kk = 0; kk < DM_BK; kk += 4) {
-            double af[8], bf[4];
-#pragma unroll
-            for (int a = 0; a < 8; ++a) af[a] = As[(kk + q) * DM_LDS + wm * 64 + a * 8 + g];
-#pragma unroll
-            for (int b = 0; b < 4; ++b) bf[b] = Bs[(kk + q) * DM_LDS + wn * 32 + b * 8 + g];
-#pragma unroll
-            for (int a = 0; a < 8; a += 2)
-#pragma unroll
-                for (int b = 0; b < 4; ++b) dmma2(acc[a][b], acc[a + 1][b], af[a], af[a + 1], bf[b]);
-        }
-        __syncthreads();
-    }
-    cp_async_wait<0>();
-
-    // epilogue: C -= acc, lower part of the region only.  The C values of two
-    // fragment rows (16 per thread) are loaded together before any store, so
-    // the loads overlap instead of serialising behind the stores.
-#pragma unroll
-    for (int a2 = 0; a2 < 8; a2 += 2) {
-        double cv[2][4][2];
-        bool ok[2][4][2];
-#pragma unroll
-        for (int h = 0; h < 2; ++h)
-#pragma unroll
-            for (int b = 0; b < 4; ++b)
-#pragma unroll
-                for (int e = 0; e < 2; ++e) {
-                    const long long i = ri + wm * 64 + (a2 + h) * 8 + g;
-                    const long long jj = rj + wn * 32 + b * 8 + 2 * q + e;
-                    ok[h][b][e] = i < n && jj < cend && i >= jj;
-                    cv[h][b][e] = ok[h][b][e] ? __ldcg(UP ? A + jj + i * lda : A + i + jj * lda) : 0.0;
-                }
-#pragma unroll
-        for (int h = 0; h < 2; ++h)
-#pragma unroll
-            for (int b = 0; b < 4; ++b)
-#pragma unroll
-                for (int e = 0; e < 2; ++e) {
-                    if (!ok[h][b][e]) continue;
-                    const long long i = ri + wm * 64 + (a2 + h) * 8 + g;
-                    const long long jj = rj + wn * 32 + b * 8 + 2 * q + e;
-                    double* p = UP ? A + jj + i * lda : A + i + jj * lda;
-                    *p = cv[h][b][e] - acc[a2 + h][b][e];
-                }
-    }
-}
-
 // ---------------------------------------------------------------------------
-// The same update with its operand slices delivered by TMA (lower storage, even
-// leading dimension, 16-byte aligned base, K a multiple of 32): per stage one
-// thread loads the A rows [ri, ri+132) and the B rows [rj, rj+132) of 32 panel
-// columns as two 132 x 32 FP64 boxes (the 4 extra rows pad the leading dimension
-// of the shared tile to 132, which keeps the fragment reads conflict free; rows
-// past n arrive as zeros), so no thread spends issue slots on per-element copies.
-// 3 stages of 66 KB.  No CTA barrier per stage: each warp releases a stage on
-// its `empty` mbarrier when done with it, and the loading thread refills the
-// stage of chunk c - 1 (long released by the other warps) after its own chunk c,
-// so the warps drift freely and the DMMA pipe is not drained once per chunk.
+// FP64 on the tensor cores (m16n8k4 DMMA), either triangle.  A CTA owns one
+// BM x BN lower tile of the region: RW x CW warps hold the accumulators; 32-column
+// slices of the panel rows [ri, ri + BM) and [rj, rj + BN) come through a ring of NS
+// stages with a `full` and an `empty` mbarrier each.  Every warp releases a stage by
+// itself and the stage of slice c - 1 is refilled after slice c, so the warps drift
+// and the DMMA pipe is not drained once per slice.
+//
+// Shared slices, in doubles (both keep the 8-byte fragment reads conflict free):
+//   'L' storage: [32 k][rows + 4]     'U' storage (k contiguous): [rows][36]
+// Two ways in:
+//   TMA  thread 0, one box per operand (4 extra rows or columns pad the slice); base
+//        16-byte aligned and even lda
+//   CP   16-byte cp.async by all threads for any lda and any 8-byte aligned base: a line (a column of 'L', a row of 'U') that starts on an odd 8-byte
+//        word is copied from one word earlier and lands one word later in its
+//        slice.  The parity alternates with the line when lda is odd, and a lane's
+//        fragments always come from lines of one parity, so the readers just add
+//        a per-lane offset.  Words past the limits are zero-filled, not read.
+// What bounds it: the DMMA pipe (FP64 tensor, 35.5 TFLOP/s by cuBLAS DGEMM); odd leading
+// dimensions cost about as much as even ones (the 16-byte copies of a slice are some 17
+// per thread against 256 DMMAs per warp).
 // Every wait is bounded: if one gives up, the CTA records it in g_dmma_status,
-// writes NaN into its tile (the factorization then stops at that column block
-// with a failed pivot) and waits, bounded, for its copies still in flight
-// before it exits.
+// writes NaN into its tile (the factorization then stops at that column block with
+// a failed pivot) and waits, bounded, for its copies still in flight.
 // ---------------------------------------------------------------------------
-constexpr int DT_BK = 32, DT_LDS = 132, DT_NS = 3;
-constexpr int DT_BOX = DT_BK * DT_LDS;                                  // doubles per operand box
-constexpr unsigned DT_BOX_BYTES = DT_BOX * 8u;                           // 33792
-constexpr size_t DT_SMEM = (size_t)DT_NS * 2 * DT_BOX_BYTES + 128;      // + alignment slack
+constexpr int SY_BK = 32;
+
+template <int BM_, int BN_, int RW_, int CW_, int NS_, int PER_SM_>
+struct SyCfg {
+    static constexpr int BM = BM_, BN = BN_, RW = RW_, CW = CW_, NS = NS_, PER_SM = PER_SM_;
+    static constexpr int WM = BM / RW, WN = BN / CW;  // a warp's tile
+    static constexpr int FM = WM / 8, FN = WN / 8;    // its 8 x 8 fragments
+    static constexpr int WARPS = RW * CW, THREADS = 32 * WARPS;
+};
+using SyBig = SyCfg<128, 128, 2, 4, 3, 1>;
+using SySmall = SyCfg<64, 64, 2, 2, 3, 2>;
+
+template <bool UP>
+__host__ __device__ constexpr int sy_ld(int rows) { return UP ? SY_BK + 4 : rows + 4; }
+template <bool UP>
+__host__ __device__ constexpr int sy_box(int rows) { return UP ? rows * sy_ld<UP>(rows) : SY_BK * sy_ld<UP>(rows); }
+template <class Cfg, bool UP>
+constexpr size_t sy_smem() { return (size_t)Cfg::NS * (sy_box<UP>(Cfg::BM) + sy_box<UP>(Cfg::BN)) * 8 + 128; }
 
 __device__ int g_dmma_status;
 
-template <bool BATCH>  // BATCH: blockIdx.y is the matrix of a batch (3-D map, matrices astride apart)
-__global__ void __launch_bounds__(256, 1) k_syrk_dmma_tma(const __grid_constant__ CUtensorMap amap,
-                                                          double* __restrict__ A, long long lda, long long astride,
-                                                          int k0, int nbk, int n, long long t0, int cols,
-                                                          const int* __restrict__ info)
+// Where the shared copy of a line starts relative to its slice row: 1 when the line's
+// first word (A + start + line * lda) is not 16-byte aligned.
+__device__ __forceinline__ int sy_shift(const double* A, long long lda, long long line, long long start)
 {
-    extern __shared__ __align__(128) unsigned char dt_raw[];
-    __shared__ __align__(8) uint64_t full[DT_NS], empty[DT_NS];
+    return (int)(((reinterpret_cast<uintptr_t>(A) >> 3) + (uintptr_t)(line * lda + start)) & 1);
+}
+
+// The CP copies of thread `t` of `nt`: `lines` lines of `len` words starting at word `start` (valid below
+// wlim; lines valid below llim), line l at A + (line0 + l) * lda, into dst + l * ld.
+__device__ __forceinline__ void sy_copy(double* dst, int ld, const double* A, long long lda, long long line0, int lines,
+                                        long long llim, long long start, int len, long long wlim, int t,
+                                        int nt)
+{
+    const int units = (len + 2) / 2;  // 16-byte units of a shifted line
+    for (int x = t; x < lines * units; x += nt) {
+        const int l = x / units, u = x - l * units;
+        const long long line = line0 + l;
+        const int sh = sy_shift(A, lda, line, start);
+        const long long w = start - sh + 2 * u;
+        const int bytes = line < llim && w < wlim ? (w + 1 < wlim ? 16 : 8) : 0;
+        cp_async16(dst + l * ld + 2 * u, bytes ? A + line * lda + w : A - ((reinterpret_cast<uintptr_t>(A) >> 3) & 1),
+                   bytes);
+    }
+}
+
+template <class Cfg, bool UP, bool TMA, bool BATCH>  // BATCH: blockIdx.y is the matrix of a batch (3-D maps)
+__global__ void __launch_bounds__(Cfg::THREADS, Cfg::PER_SM)
+    k_syrk_dmma(const __grid_constant__ CUtensorMap amap, const __grid_constant__ CUtensorMap bmap,
+                double* __restrict__ A, long long lda, long long astride, int k0, int nbk, int n, long long t0,
+                int cols, const int* __restrict__ info)
+{
+    constexpr int BM = Cfg::BM, BN = Cfg::BN, NS = Cfg::NS, FM = Cfg::FM, FN = Cfg::FN;
+    constexpr int LDA_S = sy_ld<UP>(BM), LDB_S = sy_ld<UP>(BN), ABOX = sy_box<UP>(BM), BBOX = sy_box<UP>(BN);
+    extern __shared__ __align__(128) unsigned char sy_raw[];
+    __shared__ __align__(8) uint64_t full[NS], empty[NS];
     const int z = BATCH ? (int)blockIdx.y : 0;
     A += (long long)z * astride;
     info += z;
     if (*(volatile const int*)info != 0) return;
-    int I, J;
+    int I, J;  // tile row and column, the tile's last row at or below its first column
+    const int nct = cols == 0 ? 0 : (cols + BN - 1) / BN;
     if (cols == 0) {
+        static_assert(BM == BN, "square tiles");
         tile_of_tri(blockIdx.x, I, J);
     } else {
-        const int nct = (cols + DM_BM - 1) / DM_BM;
         J = blockIdx.x % nct;
         I = blockIdx.x / nct;
         if (I < J) return;
     }
     const long long cend = cols == 0 ? (long long)n : t0 + cols;
-    const long long ri = t0 + (long long)I * DM_BM, rj = t0 + (long long)J * DM_BM;
-    double* sm = reinterpret_cast<double*>((reinterpret_cast<uintptr_t>(dt_raw) + 127) & ~uintptr_t(127));
+    const long long ri = t0 + (long long)I * BM, rj = t0 + (long long)J * BN;
+    double* sm = reinterpret_cast<double*>((reinterpret_cast<uintptr_t>(sy_raw) + 127) & ~uintptr_t(127));
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int wm = warp >> 2, wn = warp & 3;
-    const int g = lane >> 2, q = lane & 3;
-    const int nchunks = nbk / DT_BK;
-
-    auto issue = [&](int c) {
-        const int s = c % DT_NS;
-        double* st = sm + (size_t)s * 2 * DT_BOX;
-        tc::mbar_expect_tx(&full[s], 2 * DT_BOX_BYTES);
-        if (BATCH) {
-            tc::tma_load_3d(st, &amap, &full[s], (int)ri, k0 + c * DT_BK, z);
-            tc::tma_load_3d(st + DT_BOX, &amap, &full[s], (int)rj, k0 + c * DT_BK, z);
-        } else {
-            tc::tma_load_2d(st, &amap, &full[s], (int)ri, k0 + c * DT_BK);
-            tc::tma_load_2d(st + DT_BOX, &amap, &full[s], (int)rj, k0 + c * DT_BK);
-        }
-    };
+    const int nchunks = nbk / SY_BK;
     if (threadIdx.x == 0) {
-        for (int s = 0; s < DT_NS; ++s) {
-            tc::mbar_init(&full[s], 1);
-            tc::mbar_init(&empty[s], 256 / 32);  // one arrival per warp
+        for (int s = 0; s < NS; ++s) {
+            tc::mbar_init(&full[s], TMA ? 1 : Cfg::THREADS);
+            tc::mbar_init(&empty[s], Cfg::WARPS);  // one arrival per warp
         }
         tc::mbar_fence_init();
+    }
+    auto issue = [&](int c) {  // slice c into its stage: thread 0 (TMA) or every thread
+        const int s = c % NS;
+        double* st = sm + (size_t)s * (ABOX + BBOX);
+        const int kc = k0 + c * SY_BK;
+        if constexpr (TMA) {
+            tc::mbar_expect_tx(&full[s], (ABOX + BBOX) * 8u);
+            const int xa = UP ? kc : (int)ri, ya = UP ? (int)ri : kc;
+            const int xb = UP ? kc : (int)rj, yb = UP ? (int)rj : kc;
+            if (BATCH) {
+                tc::tma_load_3d(st, &amap, &full[s], xa, ya, z);
+                tc::tma_load_3d(st + ABOX, &bmap, &full[s], xb, yb, z);
+            } else {
+                tc::tma_load_2d(st, &amap, &full[s], xa, ya);
+                tc::tma_load_2d(st + ABOX, &bmap, &full[s], xb, yb);
+            }
+        } else {
+            const int t = threadIdx.x, nt = Cfg::THREADS;
+            if (UP) {
+                sy_copy(st, LDA_S, A, lda, ri, BM, n, kc, SY_BK, kc + SY_BK, t, nt);
+                sy_copy(st + ABOX, LDB_S, A, lda, rj, BN, cend, kc, SY_BK, kc + SY_BK, t, nt);
+            } else {
+                sy_copy(st, LDA_S, A, lda, kc, SY_BK, kc + SY_BK, ri, BM, n, t, nt);
+                sy_copy(st + ABOX, LDB_S, A, lda, kc, SY_BK, kc + SY_BK, rj, BN, cend, t, nt);
+            }
+            cp_async_arrive(&full[s]);
+        }
+    };
+    const bool issuer = !TMA || threadIdx.x == 0;
+    if (TMA && issuer) {  // the barriers are this thread's own: no need to wait for the others
         tc::prefetch_tmap(&amap);
-        for (int c = 0; c < DT_NS && c < nchunks; ++c) issue(c);
+        tc::prefetch_tmap(&bmap);
+        for (int c = 0; c < NS && c < nchunks; ++c) issue(c);
     }
     __syncthreads();
+    if (!TMA)
+        for (int c = 0; c < NS && c < nchunks; ++c) issue(c);
 
-    double acc[8][4][2];
+    const int wm = (warp / Cfg::CW) * Cfg::WM, wn = (warp % Cfg::CW) * Cfg::WN;
+    const int g = lane >> 2, q = lane & 3;
+    double acc[FM][FN][2];
 #pragma unroll
-    for (int a = 0; a < 8; ++a)
+    for (int a = 0; a < FM; ++a)
 #pragma unroll
-        for (int b = 0; b < 4; ++b) acc[a][b][0] = acc[a][b][1] = 0.0;
-
+        for (int b = 0; b < FN; ++b) acc[a][b][0] = acc[a][b][1] = 0.0;
+    // this lane's fragment words: row (wm + 8 a + g), k = kk + q
+    const int sha = TMA ? 0 : (UP ? sy_shift(A, lda, ri + g, k0) : sy_shift(A, lda, k0 + q, ri));
+    const int shb = TMA ? 0 : (UP ? sy_shift(A, lda, rj + g, k0) : sy_shift(A, lda, k0 + q, rj));
+    const int fa = (UP ? (wm + g) * LDA_S + q : q * LDA_S + wm + g) + sha;
+    const int fb = (UP ? (wn + g) * LDB_S + q : q * LDB_S + wn + g) + shb;
     bool ok = true;
-    int consumed = 0, issued = nchunks < DT_NS ? nchunks : DT_NS;  // issued: thread 0's count
+    int consumed = 0, issued = nchunks < NS ? nchunks : NS;
     for (int c = 0; c < nchunks; ++c) {
-        const int s = c % DT_NS;
-        if (!tc::mbar_wait(&full[s], (uint32_t)((c / DT_NS) & 1), &g_dmma_status, 0x41)) {
+        const int s = c % NS;
+        if (!tc::mbar_wait(&full[s], (uint32_t)((c / NS) & 1), &g_dmma_status, 0x41)) {
             ok = false;
             break;
         }
         consumed = c + 1;
-        const double* As = sm + (size_t)s * 2 * DT_BOX;
-        const double* Bs = As + DT_BOX;
+        const double* As = sm + (size_t)s * (ABOX + BBOX) + fa;
+        const double* Bs = sm + (size_t)s * (ABOX + BBOX) + ABOX + fb;
 #pragma unroll
-        for (int kk = 0; kk < DT_BK; kk += 4) {
-            double af[8], bf[4];
+        for (int kk = 0; kk < SY_BK; kk += 4) {
+            double af[FM], bf[FN];
 #pragma unroll
-            for (int a = 0; a < 8; ++a) af[a] = As[(kk + q) * DT_LDS + wm * 64 + a * 8 + g];
+            for (int a = 0; a < FM; ++a) af[a] = As[UP ? 8 * a * LDA_S + kk : kk * LDA_S + 8 * a];
 #pragma unroll
-            for (int b = 0; b < 4; ++b) bf[b] = Bs[(kk + q) * DT_LDS + wn * 32 + b * 8 + g];
+            for (int b = 0; b < FN; ++b) bf[b] = Bs[UP ? 8 * b * LDB_S + kk : kk * LDB_S + 8 * b];
 #pragma unroll
-            for (int a = 0; a < 8; a += 2)
+            for (int a = 0; a < FM; a += 2)
 #pragma unroll
-                for (int b = 0; b < 4; ++b) dmma2(acc[a][b], acc[a + 1][b], af[a], af[a + 1], bf[b]);
+                for (int b = 0; b < FN; ++b) dmma2(acc[a][b], acc[a + 1][b], af[a], af[a + 1], bf[b]);
         }
         __syncwarp();
         if (lane == 0) tc::mbar_arrive(&empty[s]);  // this warp is done with stage s
-        if (threadIdx.x == 0 && c >= 1 && c - 1 + DT_NS < nchunks) {
-            const int cp = c - 1;  // refill chunk cp's stage with chunk cp + NS
-            if (!tc::mbar_wait(&empty[cp % DT_NS], (uint32_t)((cp / DT_NS) & 1), &g_dmma_status, 0x44)) {
+        if (issuer && c >= 1 && c - 1 + NS < nchunks) {
+            const int cp = c - 1;  // refill slice cp's stage with slice cp + NS
+            if (!tc::mbar_wait(&empty[cp % NS], (uint32_t)((cp / NS) & 1), &g_dmma_status, 0x44)) {
                 ok = false;
                 break;
             }
-            issue(cp + DT_NS);
-            issued = cp + DT_NS + 1;
+            issue(cp + NS);
+            issued = cp + NS + 1;
         }
     }
+    if (!TMA) cp_group_wait<0>();
     ok = __syncthreads_and(ok);
-    if (!ok) {
-        // copies issued for chunks consumed .. issued - 1 may still be in flight
-        if (threadIdx.x == 0) {
+    if (TMA && !ok) {  // copies issued for slices consumed .. issued - 1 may still be in flight
+        if (threadIdx.x == 0)
             for (int c = consumed; c < issued; ++c)
-                (void)tc::mbar_wait(&full[c % DT_NS], (uint32_t)((c / DT_NS) & 1), &g_dmma_status, 0x42);
-        }
+                (void)tc::mbar_wait(&full[c % NS], (uint32_t)((c / NS) & 1), &g_dmma_status, 0x42);
         __syncthreads();
+    }
+    if (!ok) {
         const double nan = __longlong_as_double(0x7ff8000000000000LL);
 #pragma unroll
-        for (int a = 0; a < 8; ++a)
+        for (int a = 0; a < FM; ++a)
 #pragma unroll
-            for (int b = 0; b < 4; ++b) acc[a][b][0] = acc[a][b][1] = nan;
+            for (int b = 0; b < FN; ++b) acc[a][b][0] = acc[a][b][1] = nan;
     }
 
-    // epilogue: C -= acc on the lower part of the region, loads of two fragment rows batched
+    // C -= acc on the lower part of the region; the C values of two fragment rows are loaded
+    // together before any store, so the loads overlap instead of serialising behind the stores
 #pragma unroll
-    for (int a2 = 0; a2 < 8; a2 += 2) {
-        double cv[2][4][2];
-        bool in[2][4][2];
+    for (int a2 = 0; a2 < FM; a2 += 2) {
+        double cv[2][FN][2];
+        bool in[2][FN][2];
 #pragma unroll
         for (int h = 0; h < 2; ++h)
 #pragma unroll
-            for (int b = 0; b < 4; ++b)
+            for (int b = 0; b < FN; ++b)
 #pragma unroll
                 for (int e = 0; e < 2; ++e) {
-                    const long long i = ri + wm * 64 + (a2 + h) * 8 + g;
-                    const long long jj = rj + wn * 32 + b * 8 + 2 * q + e;
+                    const long long i = ri + wm + (a2 + h) * 8 + g;
+                    const long long jj = rj + wn + b * 8 + 2 * q + e;
                     in[h][b][e] = i < n && jj < cend && i >= jj;
-                    cv[h][b][e] = in[h][b][e] ? __ldcg(A + i + jj * lda) : 0.0;
+                    cv[h][b][e] = in[h][b][e] ? __ldcg(UP ? A + jj + i * lda : A + i + jj * lda) : 0.0;
                 }
 #pragma unroll
         for (int h = 0; h < 2; ++h)
 #pragma unroll
-            for (int b = 0; b < 4; ++b)
+            for (int b = 0; b < FN; ++b)
 #pragma unroll
                 for (int e = 0; e < 2; ++e) {
                     if (!in[h][b][e]) continue;
-                    const long long i = ri + wm * 64 + (a2 + h) * 8 + g;
-                    const long long jj = rj + wn * 32 + b * 8 + 2 * q + e;
-                    A[i + jj * lda] = cv[h][b][e] - acc[a2 + h][b][e];
+                    const long long i = ri + wm + (a2 + h) * 8 + g;
+                    const long long jj = rj + wn + b * 8 + 2 * q + e;
+                    *(UP ? A + jj + i * lda : A + i + jj * lda) = cv[h][b][e] - acc[a2 + h][b][e];
                 }
     }
 }
 
-// The TMA variant when its conditions hold; false (nothing launched) otherwise.
-bool launch_dmma_tma(double* A, long long lda, int k0, int nbk, int n, long long t0, int cols, const int* dinfo,
-                     cudaStream_t st, cudaError_t* err)
+template <class Cfg, bool UP, bool BATCH>
+cudaError_t launch_syrk(double* A, long long lda, long long astride, int batch, int k0, int nbk, int n, long long t0,
+                        int cols, const int* dinfo, cudaStream_t st)
 {
-    if ((lda & 1) || (reinterpret_cast<uintptr_t>(A) & 15) || (t0 & 1) || nbk % DT_BK != 0 || nbk <= 0) return false;
-    const long long m = (long long)n - t0;
-    if (m <= 0) {
-        *err = cudaSuccess;
-        return true;
+    const long long tr = ceil_div((long long)n - t0, Cfg::BM);
+    const dim3 grid((unsigned)(cols == 0 ? tr * (tr + 1) / 2 : tr * ceil_div(cols, Cfg::BN)), (unsigned)batch);
+    constexpr size_t smem = sy_smem<Cfg, UP>();
+    CUtensorMap amap{}, bmap{};
+    auto encode = [&](CUtensorMap* map, int rows) {
+        const int bx = UP ? sy_ld<UP>(rows) : rows + 4, by = UP ? rows : SY_BK;
+        if (BATCH)
+            return tc::encode_colmajor_3d(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 8, A, n, n, lda, batch, astride, bx, by);
+        return tc::encode_colmajor_2d(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 8, A, n, n, lda, bx, by,
+                                      CU_TENSOR_MAP_SWIZZLE_NONE);
+    };
+    cudaError_t e = cudaSuccess;
+    if (!(t0 & 1) && encode(&amap, Cfg::BM) && encode(&bmap, Cfg::BN)) {
+        auto* k = k_syrk_dmma<Cfg, UP, true, BATCH>;
+        if ((e = smem_optin(k, smem)) != cudaSuccess) return e;
+        k<<<grid, Cfg::THREADS, smem, st>>>(amap, bmap, A, lda, astride, k0, nbk, n, t0, cols, dinfo);
+    } else {
+        auto* k = k_syrk_dmma<Cfg, UP, false, BATCH>;
+        if ((e = smem_optin(k, smem)) != cudaSuccess) return e;
+        k<<<grid, Cfg::THREADS, smem, st>>>(amap, bmap, A, lda, astride, k0, nbk, n, t0, cols, dinfo);
     }
-    CUtensorMap amap;
-    if (!tc::encode_colmajor_2d(&amap, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 8, A, n, n, lda, DT_LDS, DT_BK,
-                                CU_TENSOR_MAP_SWIZZLE_NONE))
-        return false;
-    if ((*err = smem_optin(k_syrk_dmma_tma<false>, DT_SMEM)) != cudaSuccess) return true;
-    const long long t = ceil_div(m, DM_BM);
-    const long long grid = cols == 0 ? t * (t + 1) / 2 : t * ceil_div(cols, DM_BM);
-    k_syrk_dmma_tma<false><<<(unsigned)grid, 256, DT_SMEM, st>>>(amap, A, lda, 0, k0, nbk, n, t0, cols, dinfo);
-    *err = cudaGetLastError();
-    return true;
+    return cudaGetLastError();
 }
 
 }  // namespace
 
-// The same over a batch of equal-order matrices (blockIdx.y = matrix, astride
-// elements apart, info per matrix): the region from row / column t0, all of it
-// (cols == 0) or its first cols columns.  False (nothing launched) when the TMA
-// conditions do not hold.
-bool launch_dmma_tma_batched(double* A, long long lda, long long astride, int batch, int k0, int nbk, int n,
-                             long long t0, int cols, const int* dinfo, cudaStream_t st, cudaError_t* err)
+// Fewest 128 x 128 tiles for which they are used.  A region with fewer leaves SMs idle
+// (one such CTA per SM), and 64 x 64 tiles, two per SM, spread it: a whole factorization
+// at n = 2048 (look-ahead columns of 16 tiles) takes 0.86 against 1.98 ms, n = 5003 3.60
+// against 6.17 ms; at n = 16384 50.1 against 52.3 ms.  Lines at 74, 148, 296 and 592
+// tiles measured within 3 % of one another at every order.
+constexpr long long kSyrkBigTiles = 148;
+
+// The FP64 update of a batch of equal-order matrices (batch 1: one matrix, astride unused),
+// nbk a multiple of 32.
+template <bool UP, bool BATCH>
+static cudaError_t syrk_dmma(double* A, long long lda, long long astride, int batch, int k0, int nbk, int n,
+                             long long t0, int cols, const int* dinfo, cudaStream_t st)
 {
-    if ((lda & 1) || (astride & 1) || (reinterpret_cast<uintptr_t>(A) & 15) || (t0 & 1) || nbk % DT_BK != 0 ||
-        nbk <= 0 || batch < 1 || batch > 65535)
-        return false;
     const long long m = (long long)n - t0;
-    if (m <= 0) {
-        *err = cudaSuccess;
-        return true;
-    }
-    CUtensorMap amap;
-    if (!tc::encode_colmajor_3d(&amap, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 8, A, n, n, lda, batch, astride, DT_LDS, DT_BK))
-        return false;
-    if ((*err = smem_optin(k_syrk_dmma_tma<true>, DT_SMEM)) != cudaSuccess) return true;
-    const long long t = ceil_div(m, DM_BM);
-    const dim3 grid((unsigned)(cols == 0 ? t * (t + 1) / 2 : t * ceil_div(cols, DM_BM)), (unsigned)batch);
-    k_syrk_dmma_tma<true><<<grid, 256, DT_SMEM, st>>>(amap, A, lda, astride, k0, nbk, n, t0, cols, dinfo);
-    *err = cudaGetLastError();
-    return true;
+    if (m <= 0) return cudaSuccess;
+    if (nbk <= 0 || nbk % SY_BK != 0) return cudaErrorInvalidValue;
+    const long long t = ceil_div(m, 128);
+    const long long tiles = (cols == 0 ? t * (t + 1) / 2 : t * ceil_div(cols, 128)) * batch;
+    if (tiles < kSyrkBigTiles)
+        return launch_syrk<SySmall, UP, BATCH>(A, lda, astride, batch, k0, nbk, n, t0, cols, dinfo, st);
+    return launch_syrk<SyBig, UP, BATCH>(A, lda, astride, batch, k0, nbk, n, t0, cols, dinfo, st);
+}
+
+cudaError_t launch_syrk_batched(double* A, long long lda, long long astride, int batch, int k0, int nbk, int n,
+                                long long t0, int cols, const int* dinfo, cudaStream_t st)
+{
+    if (batch < 1 || batch > 65535) return cudaErrorInvalidValue;
+    return syrk_dmma<false, true>(A, lda, astride, batch, k0, nbk, n, t0, cols, dinfo, st);
 }
 
 namespace {
@@ -559,20 +501,6 @@ bool launch_zmma_tma(cf64* A, long long lda, int k0, int nbk, int n, long long t
     return true;
 }
 
-template <bool UP, bool VEC2>
-cudaError_t launch_dmma(double* A, long long lda, int k0, int nbk, int n, long long t0, int cols, const int* dinfo,
-                        cudaStream_t st)
-{
-    const size_t smem = DM_NSTAGE * DM_STAGE * sizeof(double);
-    if (cudaError_t e = smem_optin(k_syrk_dmma<UP, VEC2>, smem); e != cudaSuccess) return e;
-    const long long m = (long long)n - t0;
-    if (m <= 0) return cudaSuccess;
-    const long long t = ceil_div(m, DM_BM);
-    const long long grid = cols == 0 ? t * (t + 1) / 2 : t * ceil_div(cols, DM_BM);
-    k_syrk_dmma<UP, VEC2><<<(unsigned)grid, 256, smem, st>>>(A, lda, k0, nbk, n, t0, cols, dinfo);
-    return cudaGetLastError();
-}
-
 }  // namespace
 
 template <class T, bool UP>
@@ -580,11 +508,7 @@ cudaError_t trailing_update(T* A, long long lda, int k0, int nbk, int n, long lo
                             cudaStream_t st)
 {
     if constexpr (std::is_same<T, double>::value) {
-        const bool vec2 = !UP && (lda % 2 == 0) && ((reinterpret_cast<uintptr_t>(A) & 15) == 0) && (t0 % 2 == 0);
-        cudaError_t e = cudaSuccess;
-        if (vec2 && launch_dmma_tma(A, lda, k0, nbk, n, t0, cols, dinfo, st, &e)) return e;
-        if (vec2) return launch_dmma<false, true>(A, lda, k0, nbk, n, t0, cols, dinfo, st);
-        return launch_dmma<UP, false>(A, lda, k0, nbk, n, t0, cols, dinfo, st);
+        return syrk_dmma<UP, false>(A, lda, 0, 1, k0, nbk, n, t0, cols, dinfo, st);
     }
     if constexpr (std::is_same<T, cf64>::value && !UP) {
         cudaError_t e = cudaSuccess;
