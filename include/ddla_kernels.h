@@ -221,8 +221,8 @@ unsigned long long ddlak_inv_diag_bytes(int n);
 int ddlak_inv_diag_blocks(int n, const void* L32, long long ldl, void* Dinv, void* stream);
 
 /* In-place solve L L^T X = B with an FP32 factor (lower, ldl) and FP64 B;
- * scratch as ddlak_potrs_workspace(n, nrhs).  Dinv (may be NULL) holds the
- * inverted diagonal blocks; with it the diagonal steps are products. */
+ * scratch as ddlak_potrs_workspace(n, nrhs).  Dinv (may be NULL) is accepted and
+ * not read: the solve inverts its diagonal blocks itself. */
 int ddlak_potrs_mixed(int n, int nrhs, const void* L32, long long ldl, const void* Dinv, void* B, long long ldb,
                       void* work, unsigned long long work_bytes, void* stream);
 

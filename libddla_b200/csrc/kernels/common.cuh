@@ -135,6 +135,12 @@ __device__ __forceinline__ int ld_acquire(const int* p)
     asm volatile("ld.acquire.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
     return v;
 }
+__device__ __forceinline__ int ld_relaxed(const int* p)
+{
+    int v;
+    asm volatile("ld.relaxed.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
 __device__ __forceinline__ void st_release(int* p, int v)
 {
     asm volatile("st.release.gpu.global.b32 [%0], %1;" :: "l"(p), "r"(v) : "memory");
@@ -181,6 +187,12 @@ __device__ __forceinline__ void cp_async_elem(void* smem, const void* gmem, bool
     asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(s), "l"(gmem), "n"(BYTES),
                  "r"(valid ? BYTES : 0)
                  : "memory");
+}
+// 16 bytes from a 16-byte aligned address (zero-filled when !valid)
+__device__ __forceinline__ void cp_async_elem16(void* smem, const void* gmem, bool valid)
+{
+    const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(s), "l"(gmem), "r"(valid ? 16 : 0) : "memory");
 }
 __device__ __forceinline__ void cp_group_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>

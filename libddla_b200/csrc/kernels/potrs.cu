@@ -76,42 +76,23 @@ __device__ __forceinline__ T shfl_t(T v, int src)
 //   Xs[RB][RC+1]       the solved block of the other block row
 //   Acc[RB][RC+1]      this block row's right-hand sides
 //   Rinv[RB]           reciprocal pivots (real type)
-//   Ibuf[RB][RB+1]     (INV mode) the precomputed inverse of the diagonal block
-// The factor is stored as TL and the right-hand sides as TX (TL == TX on the
-// plain path; an FP32 factor with FP64 vectors for the mixed-precision solves).
-template <class TL, class TX, bool INV = false>
+template <class T>
 __host__ __device__ constexpr size_t potrs_smem_bytes()
 {
-    return sizeof(TL) * 2 * (size_t)RB * (RB + 1) + sizeof(TX) * 2 * (size_t)RB * (RC + 1) + sizeof(real_t<TX>) * RB +
-           (INV ? sizeof(TX) * (size_t)RB * (RB + 1) + 16 : 0);
+    return sizeof(T) * (2 * (size_t)RB * (RB + 1) + 2 * (size_t)RB * (RC + 1)) + sizeof(real_t<T>) * RB;
 }
 
-template <class TX, class TL>
-__device__ __forceinline__ TX widen(TL v)
-{
-    if constexpr (std::is_same<TX, TL>::value) return v;
-    else return static_cast<TX>(v);
-}
-
-// INV: the diagonal step multiplies by Dinv (TX, one RB x RB column-major block per
-// block row, entries (r, c) of inv(L_bb), zero outside the block) instead of
-// substituting; for the repeated solves of the refinement with one factor.
-// ID: forward substitution only, on the identity (generated in place of B's
-// initial values): X = L^-1.  Chunk c's columns start at row c*RC, so block
-// rows above that one are zero and are neither computed nor waited for.
-// FO: forward substitution only, on B: X = L^-1 B (side 'L') or B L^-H (side
-// 'R'); the forward half of the two-sided solve, every CTA a forward one.
-template <class TL, class TX, bool UP, bool BT, bool INV = false, bool ID = false, bool FO = false>
-__global__ void __launch_bounds__(NT) k_potrs_fused(const TL* __restrict__ A, long long lda, TX* B, long long ldb,
+// Complex types.  FO: forward substitution only, on B: X = L^-1 B (side 'L') or B L^-H
+// (side 'R'); the forward half of the two-sided solve, every CTA a forward one.
+template <class T, bool UP, bool BT, bool FO = false>
+__global__ void __launch_bounds__(NT) k_potrs_fused(const T* __restrict__ A, long long lda, T* B, long long ldb,
                                                     int n, int nrhs, int nchunks, int* flags, int* ticket,
-                                                    int* status, const TX* __restrict__ Dinv)
+                                                    int* status)
 {
-    using T = TX;
+    using TL = T;
     using R = real_t<T>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     TL (*Lbuf)[RB][RB + 1] = reinterpret_cast<TL (*)[RB][RB + 1]>(smem_raw);
-    T (*Ibuf)[RB + 1] = reinterpret_cast<T (*)[RB + 1]>(
-        smem_raw + ((potrs_smem_bytes<TL, TX, false>() + 15) / 16) * 16);
     T (*Xs)[RC + 1] = reinterpret_cast<T (*)[RC + 1]>(smem_raw + sizeof(TL) * 2 * RB * (RB + 1));
     T (*Acc)[RC + 1] = Xs + RB;
     R* Rinv = reinterpret_cast<R*>(Acc + RB);
@@ -124,13 +105,11 @@ __global__ void __launch_bounds__(NT) k_potrs_fused(const TL* __restrict__ A, lo
     const int t = s_t;
     const int chunk = t % nchunks;
     const int step = t / nchunks;
-    const bool fwd = ID || FO || step < N;
-    const int blk = ID ? step : (fwd ? step : 2 * N - 1 - step);
+    const bool fwd = FO || step < N;
+    const int blk = fwd ? step : 2 * N - 1 - step;
     int* cflags = flags + (size_t)chunk * 2 * N;  // [0,N) forward, [N,2N) backward
     const long long r0 = (long long)chunk * RC;
     const int nr = (int)((nrhs - r0) < RC ? (nrhs - r0) : RC);
-    const int jfirst = ID ? (int)(r0 / RB) : 0;  // first block row with a nonzero right-hand side
-    if (ID && blk < jfirst) return;
     const long long i0 = (long long)blk * RB;
     const int nrows = (int)((n - i0) < RB ? (n - i0) : RB);
     // raw tile element (i, k): A[(i0+i) + (j0+k)*lda] when p1, A[(j0+k) + (i0+i)*lda] otherwise;
@@ -143,8 +122,8 @@ __global__ void __launch_bounds__(NT) k_potrs_fused(const TL* __restrict__ A, lo
 
     // Visit the other block rows in publication order (forward 0, 1, ..; backward N-1, N-2, ..):
     // every wait but the last one is already satisfied when reached.
-    const int nvisit = ID ? blk - jfirst : (fwd ? blk : N - 1 - blk);
-    auto visit = [&](int v) { return ID ? jfirst + v : (fwd ? v : N - 1 - v); };
+    const int nvisit = fwd ? blk : N - 1 - blk;
+    auto visit = [&](int v) { return fwd ? v : N - 1 - v; };
     auto issue_tile = [&](int j, int buf) {
         const long long j0 = (long long)j * RB;
         const int ncols = (int)((n - j0) < RB ? (n - j0) : RB);
@@ -161,14 +140,6 @@ __global__ void __launch_bounds__(NT) k_potrs_fused(const TL* __restrict__ A, lo
     // L(r, c) = D[c][r] ('L') or conj(D[c][r]) ('U') for r >= c.  Prefetched into the ring slot
     // the last off-diagonal tile leaves free, so it is resident when the solve reaches it.
     auto issue_diag = [&](int buf) {
-        if constexpr (INV) {
-            const T* src0 = Dinv + (long long)blk * RB * RB;
-            for (int idx = threadIdx.x; idx < RB * RB; idx += NT) {
-                const int r = idx % RB, c = idx / RB;
-                cp_async_elem<sizeof(T)>(&Ibuf[c][r], src0 + idx, true);
-            }
-            return;
-        }
         for (int idx = threadIdx.x; idx < RB * RB; idx += NT) {
             int r, c;
             const TL* src;
@@ -194,10 +165,7 @@ __global__ void __launch_bounds__(NT) k_potrs_fused(const TL* __restrict__ A, lo
 #pragma unroll
     for (int q = 0; q < RC / 4; ++q) {
         const int r = tg + 4 * q;
-        if constexpr (ID)
-            acc[q] = (tr < nrows && r < nr && i0 + tr == r0 + r) ? from_real<T>(R(1)) : zero<T>();
-        else
-            acc[q] = (tr < nrows && r < nr) ? x_ld_cg<T, BT>(B, ldb, i0 + tr, r0 + r) : zero<T>();
+        acc[q] = (tr < nrows && r < nr) ? x_ld_cg<T, BT>(B, ldb, i0 + tr, r0 + r) : zero<T>();
     }
 
     // The solved block of the next visit is fetched into registers (L2 loads) while
@@ -252,14 +220,14 @@ __global__ void __launch_bounds__(NT) k_potrs_fused(const TL* __restrict__ A, lo
         if (p1) {
 #pragma unroll 8
             for (int k = 0; k < RB; ++k) {
-                const T l = widen<T>(Lt[k][tr]);
+                const T l = Lt[k][tr];
 #pragma unroll
                 for (int q = 0; q < RC / 4; ++q) acc[q] = fms(acc[q], l, Xs[k][tg + 4 * q]);
             }
         } else {
 #pragma unroll 8
             for (int k = 0; k < RB; ++k) {
-                const T l = cj(widen<T>(Lt[k][tr]));
+                const T l = cj(Lt[k][tr]);
 #pragma unroll
                 for (int q = 0; q < RC / 4; ++q) acc[q] = fms(acc[q], l, Xs[k][tg + 4 * q]);
             }
@@ -270,39 +238,14 @@ __global__ void __launch_bounds__(NT) k_potrs_fused(const TL* __restrict__ A, lo
 
     const TL (*D)[RB + 1] = Lbuf[nvisit & 1];
     // L(r, c) for r >= c, and conj(L(c, r)) for c > r, from the raw diagonal block
-    auto lval = [&](int r, int c) { return UP ? cj(widen<T>(D[c][r])) : widen<T>(D[c][r]); };
-    auto lcval = [&](int c, int r) { return UP ? widen<T>(D[r][c]) : cj(widen<T>(D[r][c])); };
+    auto lval = [&](int r, int c) { return UP ? cj(D[c][r]) : D[c][r]; };
+    auto lcval = [&](int c, int r) { return UP ? D[r][c] : cj(D[r][c]); };
 #pragma unroll
     for (int q = 0; q < RC / 4; ++q) Acc[tr][tg + 4 * q] = acc[q];
     __syncthreads();
-    if constexpr (!INV)
-        for (int k = threadIdx.x; k < RB; k += NT) Rinv[k] = k < nrows ? R(1) / re(widen<T>(D[k][k])) : R(0);
+    for (int k = threadIdx.x; k < RB; k += NT) Rinv[k] = k < nrows ? R(1) / re(D[k][k]) : R(0);
     __syncthreads();
-    if constexpr (INV) {
-        // diagonal step as a product with the precomputed inverse block:
-        // forward x = inv(L_bb) acc, backward x = inv(L_bb)^H acc
-        T out[RC / 4];
-#pragma unroll
-        for (int q = 0; q < RC / 4; ++q) out[q] = zero<T>();
-        if (fwd) {
-#pragma unroll 8
-            for (int k = 0; k < RB; ++k) {
-                const T m = Ibuf[k][tr];
-#pragma unroll
-                for (int q = 0; q < RC / 4; ++q) out[q] = fma_(out[q], m, Acc[k][tg + 4 * q]);
-            }
-        } else {
-#pragma unroll 8
-            for (int k = 0; k < RB; ++k) {
-                const T m = cj(Ibuf[tr][k]);
-#pragma unroll
-                for (int q = 0; q < RC / 4; ++q) out[q] = fma_(out[q], m, Acc[k][tg + 4 * q]);
-            }
-        }
-        __syncthreads();
-#pragma unroll
-        for (int q = 0; q < RC / 4; ++q) Acc[tr][tg + 4 * q] = out[q];
-    } else {
+    {
         // warp w solves right-hand sides 2w and 2w+1 together; lanes own rows lane and lane+32
         const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
         const int ra = 2 * warp, rb = 2 * warp + 1;
@@ -369,22 +312,330 @@ __global__ void __launch_bounds__(NT) k_potrs_fused(const TL* __restrict__ A, lo
     if (threadIdx.x == 0) st_release(&cflags[fwd ? blk : N + blk], 1);
 }
 
-template <class T, bool UP, bool BT, class TL = T, bool INV = false, bool ID = false, bool FO = false>
+// ---------------------------------------------------------------------------
+// The same solve for real types on the FP64 tensor cores (m16n8k4 DMMA, FP64
+// arithmetic for FP32 and FP64 storage).  Eight warps: warp w owns rows
+// 16 (w % 4) .. + 15 of the block row and right-hand sides 8 (w / 4) .. + 7 of the
+// chunk, as one accumulator fragment.
+//   * Before it joins the chain, a CTA inverts its 64 x 64 diagonal block (8 x 8
+//     tiles by substitution, then the identity's 16-row strips against the block,
+//     as the panel solve of panel.cu), so a link of the chain is two products
+//     (the last off-diagonal tile, the inverse) and no substitution.
+//   * One thread polls the flag of the block needed; every warp reads that block's
+//     solution straight into its operand fragments; the next one is fetched under
+//     the current product when its flag is already up.
+// What bounds it: the chain of n / 64 links per direction.  Measured (factor and flags
+// in place, one call): n = 2048, 16 right-hand sides 345 against 556 us for the
+// substitution form, n = 5003, 3 of them 0.88 against 1.38 ms; n = 16384, 64 of them
+// 6.6 ms either way.
+// ---------------------------------------------------------------------------
+constexpr int PD_LD = RB + 4;  // 4 mod 16 doubles: conflict-free fragment reads either way round
+constexpr int PD_LDX = RC + 4;
+
+template <class TL>
+__host__ __device__ constexpr size_t potrs_dmma_smem()
+{
+    return 2 * (size_t)RB * PD_LD * sizeof(TL) + (size_t)RB * PD_LD * sizeof(double) +
+           (sizeof(TL) < 8 ? (size_t)RB * PD_LDX * sizeof(double) : 0);
+}
+
+__device__ __forceinline__ void pd_mma(double (&d)[4], double a_up, double a_lo, double b)
+{
+    asm volatile("mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};"
+                 : "+d"(d[0]), "+d"(d[1]), "+d"(d[2]), "+d"(d[3])
+                 : "d"(a_up), "d"(a_lo), "d"(b));
+}
+
+// One thread: until *flag >= 1 or the budget runs out (DDLAK_WAIT_TIMEOUT in *status, false).
+// Relaxed polls and one fence: an acquire per poll would invalidate L1 each time.
+__device__ __forceinline__ bool poll_flag(const int* flag, int* status, bool near)
+{
+    const long long t0 = clock64(), budget = wait_budget_cycles();
+    for (unsigned it = 0;; ++it) {
+        if (ld_relaxed(flag) >= 1) {
+            __threadfence();
+            return true;
+        }
+        if ((it & 31) == 31) {
+            if (ld_relaxed(status) != DDLAK_OK) return false;
+            if (clock64() - t0 > budget) {
+                atomicCAS(status, DDLAK_OK, DDLAK_WAIT_TIMEOUT);
+                return false;
+            }
+        }
+        if (!near) __nanosleep(200);
+    }
+}
+
+template <class TL, class TX, bool UP, bool BT, bool ID, bool FO>
+__global__ void __launch_bounds__(NT, 2) k_potrs_dmma(const TL* __restrict__ A, long long lda, TX* B, long long ldb,
+                                                      int n, int nrhs, int nchunks, int* flags, int* ticket,
+                                                      int* status)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    TL* Lb = reinterpret_cast<TL*>(smem_raw);  // two tiles of RB lines of PD_LD
+    double* Ib = reinterpret_cast<double*>(smem_raw + 2 * (size_t)RB * PD_LD * sizeof(TL));  // inverse, row-major
+    // the block row's right-hand sides between the two products: over the (then free) tiles
+    double* Xs = sizeof(TL) < 8 ? Ib + RB * PD_LD : reinterpret_cast<double*>(smem_raw);
+    __shared__ __align__(16) double T8[8 * 64];  // inverses of the diagonal 8 x 8 tiles
+    __shared__ int s_t, s_next;
+    if (threadIdx.x == 0) s_t = atomicAdd(ticket, 1);
+    __syncthreads();
+    const int N = (int)ceil_div(n, RB);
+    const int t = s_t;
+    const int chunk = t % nchunks;
+    const int step = t / nchunks;
+    const bool fwd = ID || FO || step < N;
+    const int blk = ID ? step : (fwd ? step : 2 * N - 1 - step);
+    int* cflags = flags + (size_t)chunk * 2 * N;  // [0,N) forward, [N,2N) backward
+    const long long r0 = (long long)chunk * RC;
+    const int jfirst = ID ? (int)(r0 / RB) : 0;  // first block row with a nonzero right-hand side
+    if (ID && blk < jfirst) return;
+    const long long i0 = (long long)blk * RB;
+    const int nrows = (int)((n - i0) < RB ? (n - i0) : RB);
+    // operator entry (i, k) of a tile: A[(i0+i) + (j0+k)*lda] when p1, A[(j0+k) + (i0+i)*lda] otherwise
+    const bool p1 = (fwd != UP);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int g = lane >> 2, q = lane & 3;
+    const int row = 16 * (warp & 3) + g;              // and row + 8
+    const long long rc = r0 + 8 * (warp >> 2);         // this warp's first right-hand side
+    const bool live = rc < nrhs;                       // uniform over the warp
+
+    const int nvisit = ID ? blk - jfirst : (fwd ? blk : N - 1 - blk);
+    auto visit = [&](int v) { return ID ? jfirst + v : (fwd ? v : N - 1 - v); };
+    // tile lines: p1 [k][i], otherwise [i][k]; the line's words are contiguous in A
+    auto issue_tile = [&](int j, int buf) {
+        const long long j0 = (long long)j * RB;
+        const int ncols = (int)((n - j0) < RB ? (n - j0) : RB);
+        TL* dst = Lb + buf * RB * PD_LD;
+        const TL* src0 = p1 ? A + i0 + j0 * lda : A + j0 + i0 * lda;
+        const int wlim = p1 ? nrows : ncols, llim = p1 ? ncols : nrows;
+        if (sizeof(TL) == 8 && !(lda & 1) && !(reinterpret_cast<uintptr_t>(A) & 15) && wlim == RB) {
+            for (int idx = threadIdx.x; idx < RB * RB / 2; idx += NT) {
+                const int l = idx >> 5, w = 2 * (idx & 31);
+                const bool in = l < llim;
+                cp_async_elem16(dst + l * PD_LD + w, in ? src0 + l * lda + w : A, in);
+            }
+        } else {
+            for (int idx = threadIdx.x; idx < RB * RB; idx += NT) {
+                const int l = idx >> 6, w = idx & (RB - 1);
+                const bool in = l < llim && w < wlim;
+                cp_async_elem<sizeof(TL)>(dst + l * PD_LD + w, in ? src0 + l * lda + w : A, in);
+            }
+        }
+    };
+    // the diagonal block into tile 0: lines [c][r] ('L') or [r][c] ('U'); its strict upper part is not used
+    {
+        const TL* src0 = A + i0 + i0 * lda;
+        for (int idx = threadIdx.x; idx < RB * RB; idx += NT) {
+            const int l = idx >> 6, w = idx & (RB - 1);
+            const bool in = l < nrows && w < nrows && (UP ? w <= l : w >= l);
+            cp_async_elem<sizeof(TL)>(Lb + l * PD_LD + w, in ? src0 + l * lda + w : A, in);
+        }
+    }
+    cp_commit();
+    if (nvisit > 0) issue_tile(visit(0), 1);
+    cp_commit();
+
+    // ---- inverse of the diagonal block (padded with the identity) --------------------
+    auto lval = [&](int r, int c) { return (double)(UP ? Lb[r * PD_LD + c] : Lb[c * PD_LD + r]); };
+    cp_wait<1>();
+    for (int idx = threadIdx.x; idx < RB * PD_LD; idx += NT) Ib[idx] = 0.0;
+    __syncthreads();
+    if (threadIdx.x < 64) {
+        // column c of diagonal tile b's inverse
+        const int b = threadIdx.x >> 3, c = threadIdx.x & 7;
+        double y[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            double v = i == c ? 1.0 : 0.0;
+#pragma unroll
+            for (int k = 0; k < i; ++k) v = fma(-lval(8 * b + i, 8 * b + k), y[k], v);
+            y[i] = 8 * b + i < nrows ? v / lval(8 * b + i, 8 * b + i) : v;
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) T8[b * 64 + i * 8 + c] = y[i];
+    }
+    __syncthreads();
+    if (warp < 4) {
+        // X L^T = I by 16-row strips (panel.cu): X(i, m) = (L^-1)(m, i)
+        double C[8][4];
+#pragma unroll
+        for (int l = 0; l < 8; ++l)
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) C[l][2 * h + e] = row + 8 * h == 8 * l + 2 * q + e ? 1.0 : 0.0;
+#pragma unroll 1
+        for (int j = 0; j < 8; ++j) {
+            double X[4] = {0.0, 0.0, 0.0, 0.0};
+            pd_mma(X, C[0][0], C[0][2], T8[j * 64 + g * 8 + 2 * q]);
+            pd_mma(X, C[0][1], C[0][3], T8[j * 64 + g * 8 + 2 * q + 1]);
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) Ib[(8 * j + 2 * q + e) * PD_LD + row + 8 * h] = X[2 * h + e];
+#pragma unroll
+            for (int l = 1; l < 8; ++l) {
+                if (l > 7 - j) break;
+                double D[4] = {C[l][0], C[l][1], C[l][2], C[l][3]};
+                pd_mma(D, -X[0], -X[2], lval(8 * (j + l) + g, 8 * j + 2 * q));
+                pd_mma(D, -X[1], -X[3], lval(8 * (j + l) + g, 8 * j + 2 * q + 1));
+#pragma unroll
+                for (int e = 0; e < 4; ++e) C[l - 1][e] = D[e];
+            }
+        }
+    }
+    __syncthreads();
+
+    // ---- the block row -------------------------------------------------------------------
+    // one thread waits for a block's solution; the CTA learns of it at the next barrier.  A wait
+    // that is not the block row's last polls rarely: hundreds of CTAs wait at a time, and
+    // their polls of one word would delay the publication itself.
+    bool fail = false;
+    auto wait_flag = [&](const int* f, bool near) {
+        if (threadIdx.x == 0) fail = !poll_flag(f, status, near);
+        fail = __syncthreads_or(fail);
+    };
+    if (!fwd) wait_flag(&cflags[blk], nvisit == 0);  // the block row's own forward result
+    if (fail) {
+        cp_wait<0>();
+        return;
+    }
+    double acc[4], acc2[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const long long i = i0 + row + 8 * h, r = rc + 2 * q + e;
+            if (ID) acc[2 * h + e] = i == r && i < n ? 1.0 : 0.0;
+            else acc[2 * h + e] = row + 8 * h < nrows && r < nrhs ? (double)x_ld_cg<TX, BT>(B, ldb, i, r) : 0.0;
+        }
+    double xr[RB / 4];  // operand fragments of the other block's solution: X(k = 4 m + q, r = g), negated
+    bool pre = false;
+    auto load_x = [&](int j) {
+        const long long j0 = (long long)j * RB;
+#pragma unroll
+        for (int m = 0; m < RB / 4; ++m) {
+            const long long k = j0 + 4 * m + q;
+            xr[m] = k < n && rc + g < nrhs ? -(double)x_ld_cg<TX, BT>(B, ldb, k, rc + g) : 0.0;
+        }
+    };
+    for (int v = 0; v < nvisit; ++v) {
+        if (v + 1 < nvisit) issue_tile(visit(v + 1), v & 1);  // tile v sits in buffer (v + 1) & 1
+        cp_commit();
+        if (!pre) {
+            const int j = visit(v);
+            wait_flag(&cflags[fwd ? j : N + j], v + 1 == nvisit);
+            if (fail) {
+                cp_wait<0>();
+                return;
+            }
+            if (live) load_x(j);
+        }
+        if (threadIdx.x == 0) {
+            bool up = false;
+            if (v + 1 < nvisit) {
+                const int j = visit(v + 1);
+                up = ld_relaxed(&cflags[fwd ? j : N + j]) >= 1;
+                if (up) __threadfence();
+            }
+            s_next = up;
+        }
+        cp_wait<1>();
+        __syncthreads();
+        pre = s_next != 0;
+        if (live) {
+            double b[RB / 4];
+#pragma unroll
+            for (int m = 0; m < RB / 4; ++m) b[m] = xr[m];
+            if (pre) load_x(visit(v + 1));
+            const TL* Lt = Lb + ((v + 1) & 1) * RB * PD_LD;
+            if (p1) {
+#pragma unroll
+                for (int m = 0; m < RB / 4; m += 2) {
+                    const TL* p = Lt + (4 * m + q) * PD_LD + row;
+                    pd_mma(acc, (double)p[0], (double)p[8], b[m]);
+                    pd_mma(acc2, (double)p[4 * PD_LD], (double)p[4 * PD_LD + 8], b[m + 1]);
+                }
+            } else {
+#pragma unroll
+                for (int m = 0; m < RB / 4; m += 2) {
+                    const TL* p = Lt + row * PD_LD + 4 * m + q;
+                    pd_mma(acc, (double)p[0], (double)p[8 * PD_LD], b[m]);
+                    pd_mma(acc2, (double)p[4], (double)p[8 * PD_LD + 4], b[m + 1]);
+                }
+            }
+        }
+        __syncthreads();  // the tile is free
+    }
+    cp_wait<0>();
+    {
+        double* p = Xs + row * PD_LDX + 8 * (warp >> 2) + 2 * q;
+        p[0] = acc[0] + acc2[0];
+        p[1] = acc[1] + acc2[1];
+        p[8 * PD_LDX] = acc[2] + acc2[2];
+        p[8 * PD_LDX + 1] = acc[3] + acc2[3];
+    }
+    __syncthreads();
+    if (live) {
+        // x = Inv acc (forward) or Inv^T acc (backward); Inv is zero above its diagonal
+        double x[4] = {0.0, 0.0, 0.0, 0.0}, x2[4] = {0.0, 0.0, 0.0, 0.0};
+        const double* xb = Xs + 8 * (warp >> 2) + g;
+        const int s = warp & 3;
+        if (fwd) {
+#pragma unroll
+            for (int m = 0; m < RB / 4; m += 2) {
+                if (m >= 4 * (s + 1)) break;
+                const double* p = Ib + row * PD_LD + 4 * m + q;
+                pd_mma(x, p[0], p[8 * PD_LD], xb[(4 * m + q) * PD_LDX]);
+                pd_mma(x2, p[4], p[8 * PD_LD + 4], xb[(4 * m + 4 + q) * PD_LDX]);
+            }
+        } else {
+#pragma unroll
+            for (int m = 0; m < RB / 4; m += 2) {
+                if (m < 4 * s) continue;
+                const double* p = Ib + (4 * m + q) * PD_LD + row;
+                pd_mma(x, p[0], p[8], xb[(4 * m + q) * PD_LDX]);
+                pd_mma(x2, p[4 * PD_LD], p[4 * PD_LD + 8], xb[(4 * m + 4 + q) * PD_LDX]);
+            }
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const long long r = rc + 2 * q + e;
+                if (row + 8 * h < nrows && r < nrhs)
+                    x_st<TX, BT>(B, ldb, i0 + row + 8 * h, r, (TX)(x[2 * h + e] + x2[2 * h + e]));
+            }
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) st_release(&cflags[fwd ? blk : N + blk], 1);  // orders the CTA's stores too
+}
+
+template <class T, bool UP, bool BT, class TL = T, bool ID = false, bool FO = false>
 cudaError_t potrs_launch(const TL* A, long long lda, T* B, long long ldb, int n, int nrhs, int* flags, int* ticket,
-                         int* status, cudaStream_t st, const T* Dinv = nullptr)
+                         int* status, cudaStream_t st)
 {
     const int N = (int)ceil_div(n, RB);
     const int nchunks = (int)ceil_div(nrhs, RC);
     const long long grid = (ID || FO ? 1LL : 2LL) * N * nchunks;
-    const size_t smem = potrs_smem_bytes<TL, T, INV>();
-    if (cudaError_t e = smem_optin(k_potrs_fused<TL, T, UP, BT, INV, ID, FO>, smem); e != cudaSuccess) return e;
     const double cf = Traits<T>::cplx ? 4.0 : 1.0;
     const double nd = n, rd = nrhs;
     ProfScope ps(PK_POTRS_FUSED, st,
                  ID ? cf * nd * nd * nd / 3.0 : (FO ? cf * nd * nd * rd : cf * 2.0 * nd * nd * rd),
                  sizeof(TL) * nd * (nd + 1) + sizeof(T) * 4.0 * nd * rd);
-    k_potrs_fused<TL, T, UP, BT, INV, ID, FO><<<(unsigned)grid, NT, smem, st>>>(A, lda, B, ldb, n, nrhs, nchunks,
-                                                                                 flags, ticket, status, Dinv);
+    if constexpr (Traits<T>::cplx) {
+        const size_t smem = potrs_smem_bytes<T>();
+        if (cudaError_t e = smem_optin(k_potrs_fused<T, UP, BT, FO>, smem); e != cudaSuccess) return e;
+        k_potrs_fused<T, UP, BT, FO><<<(unsigned)grid, NT, smem, st>>>(A, lda, B, ldb, n, nrhs, nchunks, flags, ticket,
+                                                                       status);
+    } else {
+        const size_t smem = potrs_dmma_smem<TL>();
+        if (cudaError_t e = smem_optin(k_potrs_dmma<TL, T, UP, BT, ID, FO>, smem); e != cudaSuccess) return e;
+        k_potrs_dmma<TL, T, UP, BT, ID, FO><<<(unsigned)grid, NT, smem, st>>>(A, lda, B, ldb, n, nrhs, nchunks, flags,
+                                                                              ticket, status);
+    }
     note_launches(1);
     return cudaGetLastError();
 }
@@ -410,12 +661,12 @@ cudaError_t forward_typed(char uplo, char side, int n, int nrhs, const void* A, 
     T* b = static_cast<T*>(B);
     const bool up = uplo == 'U', bt = side == 'R';
     if (up && bt)
-        return potrs_launch<T, true, true, T, false, false, true>(a, lda, b, ldb, n, nrhs, flags, ticket, status, st);
+        return potrs_launch<T, true, true, T, false, true>(a, lda, b, ldb, n, nrhs, flags, ticket, status, st);
     if (up)
-        return potrs_launch<T, true, false, T, false, false, true>(a, lda, b, ldb, n, nrhs, flags, ticket, status, st);
+        return potrs_launch<T, true, false, T, false, true>(a, lda, b, ldb, n, nrhs, flags, ticket, status, st);
     if (bt)
-        return potrs_launch<T, false, true, T, false, false, true>(a, lda, b, ldb, n, nrhs, flags, ticket, status, st);
-    return potrs_launch<T, false, false, T, false, false, true>(a, lda, b, ldb, n, nrhs, flags, ticket, status, st);
+        return potrs_launch<T, false, true, T, false, true>(a, lda, b, ldb, n, nrhs, flags, ticket, status, st);
+    return potrs_launch<T, false, false, T, false, true>(a, lda, b, ldb, n, nrhs, flags, ticket, status, st);
 }
 
 cudaError_t potrs_dispatch(char type, char uplo, char side, int n, int nrhs, const void* A, long long lda, void* B,
@@ -512,11 +763,7 @@ extern "C" int ddlak_potrs_mixed(int n, int nrhs, const void* L32, long long ldl
     if (e != cudaSuccess) return (int)e;
     int* status = static_cast<int*>(work);
     int* flags = reinterpret_cast<int*>(static_cast<char*>(work) + 256);
-    if (Dinv)
-        return (int)potrs_launch<double, false, false, float, true>(static_cast<const float*>(L32), ldl,
-                                                                    static_cast<double*>(B), ldb, n, nrhs, flags,
-                                                                    status + 1, status, st,
-                                                                    static_cast<const double*>(Dinv));
+    (void)Dinv;  // accepted; the solve inverts the diagonal blocks itself
     return (int)potrs_launch<double, false, false, float>(static_cast<const float*>(L32), ldl,
                                                           static_cast<double*>(B), ldb, n, nrhs, flags, status + 1,
                                                           status, st);
@@ -657,10 +904,10 @@ extern "C" int ddlak_trtri_blocked(char type, int n, const void* L, long long ld
     int* ticket = status + 1;
     int* flags = reinterpret_cast<int*>(static_cast<char*>(work) + 256);
     if (type == 'd')
-        return (int)potrs_launch<double, false, false, double, false, true>(
+        return (int)potrs_launch<double, false, false, double, true>(
             static_cast<const double*>(L), ldl, static_cast<double*>(W), ldw, n, n, flags, ticket, status, st);
     if (type == 's')
-        return (int)potrs_launch<float, false, false, float, false, true>(
+        return (int)potrs_launch<float, false, false, float, true>(
             static_cast<const float*>(L), ldl, static_cast<float*>(W), ldw, n, n, flags, ticket, status, st);
     return (int)cudaErrorInvalidValue;
 }
