@@ -28,6 +28,7 @@
 
 #include "common.cuh"
 #include "profile.h"
+#include "sgemm.cuh"
 #include "tc_common.cuh"
 
 namespace ddlak {
@@ -218,6 +219,75 @@ __device__ __forceinline__ void tile_of_lower(int t, int& ti, int& tj)
     tj = t - i * (i + 1) / 2;
 }
 
+// The epilogue of a contraction tile: thread results acc[u][v] = (A^-1)(row(u), col(v)).
+// MODE 1 writes the dense adjoint, MODE 0 contracts it with dA/dtheta into partial[0..2]
+// of this tile (FP64).  All threads of the CTA; al, x, th: this matrix's.
+template <class T, int MODE, class Row, class Col>
+__device__ __forceinline__ void contract_epilogue(int n, const T (&acc)[8][8], Row row, Col col, int i0, int j0,
+                                                  const T* __restrict__ al, const T* __restrict__ x, int d,
+                                                  const double* __restrict__ th, double (*red)[CT_NT / 32],
+                                                  double* __restrict__ partial, T* __restrict__ g, long long ldg)
+{
+    const int t = threadIdx.x;
+    if constexpr (MODE == 1) {
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+#pragma unroll
+            for (int v = 0; v < 8; ++v) {
+                const int i = i0 + row(u), j = j0 + col(v);
+                if (i < n && j <= i) {
+                    const T ab = T(0.5) * (acc[u][v] - al[i] * al[j]);
+                    g[i + (long long)j * ldg] = ab;
+                    g[j + (long long)i * ldg] = ab;
+                }
+            }
+    } else {
+        const double l = th[0], sf2 = th[1];
+        const double inv2l2 = 0.5 / (l * l), invl3 = 1.0 / (l * l * l);
+        double g0 = 0.0, g1 = 0.0, g2 = 0.0;
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            const int i = i0 + row(u);
+            if (i >= n) continue;
+            const double ai = (double)al[i];
+#pragma unroll
+            for (int v = 0; v < 8; ++v) {
+                const int j = j0 + col(v);
+                if (j <= i) {
+                    const double ab = 0.5 * ((double)acc[u][v] - ai * (double)al[j]);
+                    const double w = i == j ? 1.0 : 2.0;
+                    double r2 = 0.0;
+                    for (int c = 0; c < d; ++c) {
+                        const double dx = (double)x[(long long)i * d + c] - (double)x[(long long)j * d + c];
+                        r2 += dx * dx;
+                    }
+                    const double e = exp(-r2 * inv2l2);
+                    g0 += w * ab * sf2 * e * r2 * invl3;  // dA/dl
+                    g1 += w * ab * e;                     // dA/dsigma_f^2
+                    if (i == j) g2 += ab;                 // dA/dsigma^2
+                }
+            }
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            g0 += __shfl_xor_sync(0xffffffffu, g0, o);
+            g1 += __shfl_xor_sync(0xffffffffu, g1, o);
+            g2 += __shfl_xor_sync(0xffffffffu, g2, o);
+        }
+        if ((t & 31) == 0) {
+            red[0][t >> 5] = g0;
+            red[1][t >> 5] = g1;
+            red[2][t >> 5] = g2;
+        }
+        __syncthreads();
+        if (t < 3) {
+            double sum = 0.0;
+            for (int w = 0; w < CT_NT / 32; ++w) sum += red[t][w];
+            partial[t] = sum;
+        }
+    }
+}
+
 template <class T, int MODE, bool DIRECT>
 __global__ void __launch_bounds__(CT_NT, 1)
     k_adjoint_contract(int n, const T* __restrict__ Wg, long long ldw, long long wstride,
@@ -311,67 +381,9 @@ __global__ void __launch_bounds__(CT_NT, 1)
     }
     cp_group_wait<0>();
 
-    const T* al = alpha_g + m * astride;
-    if constexpr (MODE == 1) {
-        T* g = G + m * gstride;
-#pragma unroll
-        for (int u = 0; u < 8; ++u)
-#pragma unroll
-            for (int v = 0; v < 8; ++v) {
-                const int i = i0 + row_of(u), j = j0 + col_of(v);
-                if (i < n && j <= i) {
-                    const T ab = T(0.5) * (acc[u][v] - al[i] * al[j]);
-                    g[i + (long long)j * ldg] = ab;
-                    g[j + (long long)i * ldg] = ab;
-                }
-            }
-    } else {
-        const double* th = theta + (long long)m * tstride;
-        const double l = th[0], sf2 = th[1];
-        const double inv2l2 = 0.5 / (l * l), invl3 = 1.0 / (l * l * l);
-        const T* x = X + m * xstride;
-        double g0 = 0.0, g1 = 0.0, g2 = 0.0;
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-            const int i = i0 + row_of(u);
-            if (i >= n) continue;
-            const double ai = (double)al[i];
-#pragma unroll
-            for (int v = 0; v < 8; ++v) {
-                const int j = j0 + col_of(v);
-                if (j <= i) {
-                    const double ab = 0.5 * ((double)acc[u][v] - ai * (double)al[j]);
-                    const double w = i == j ? 1.0 : 2.0;
-                    double r2 = 0.0;
-                    for (int c = 0; c < d; ++c) {
-                        const double dx = (double)x[(long long)i * d + c] - (double)x[(long long)j * d + c];
-                        r2 += dx * dx;
-                    }
-                    const double e = exp(-r2 * inv2l2);
-                    g0 += w * ab * sf2 * e * r2 * invl3;  // dA/dl
-                    g1 += w * ab * e;                     // dA/dsigma_f^2
-                    if (i == j) g2 += ab;                 // dA/dsigma^2
-                }
-            }
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            g0 += __shfl_xor_sync(0xffffffffu, g0, o);
-            g1 += __shfl_xor_sync(0xffffffffu, g1, o);
-            g2 += __shfl_xor_sync(0xffffffffu, g2, o);
-        }
-        if ((t & 31) == 0) {
-            red[0][t >> 5] = g0;
-            red[1][t >> 5] = g1;
-            red[2][t >> 5] = g2;
-        }
-        __syncthreads();
-        if (t < 3) {
-            double sum = 0.0;
-            for (int w = 0; w < CT_NT / 32; ++w) sum += red[t][w];
-            partial[((long long)m * gridDim.x + tile) * 3 + t] = sum;
-        }
-    }
+    contract_epilogue<T, MODE>(n, acc, row_of, col_of, i0, j0, alpha_g + m * astride, X + m * xstride, d,
+                               theta + (long long)m * tstride, red, partial + ((long long)m * gridDim.x + tile) * 3,
+                               G + m * gstride, ldg);
 }
 
 // out[m] = sum_i x_m[i] y_m[i] in FP64, one CTA per vector
@@ -413,14 +425,29 @@ __global__ void k_batched_logdiag(int n, const T* __restrict__ L, long long ldl,
     }
 }
 
-// grad[m][c] = sum over tiles of partial[m][tile][c], in tile order
-__global__ void k_adjoint_reduce(int ntiles, const double* __restrict__ partial, double* __restrict__ grad)
+// grad[m][c] = sum over tiles of partial[m][tile][c]: each thread a strided share in tile
+// order, then the shares pairwise in a fixed tree (the same sum every run).  One thread per
+// component took a load's latency per tile, over a millisecond for the 8256 tiles of n = 16384.
+constexpr int RD_NT = 256;
+__global__ void __launch_bounds__(RD_NT) k_adjoint_reduce(int ntiles, const double* __restrict__ partial,
+                                                          double* __restrict__ grad)
 {
-    const int m = blockIdx.x, c = threadIdx.x;
-    if (c >= 3) return;
-    double s = 0.0;
-    for (int k = 0; k < ntiles; ++k) s += partial[((long long)m * ntiles + k) * 3 + c];
-    grad[(long long)m * 3 + c] = s;
+    __shared__ double s[3][RD_NT];
+    const int m = blockIdx.x, t = threadIdx.x;
+    double a[3] = {0.0, 0.0, 0.0};
+    for (int k = t; k < ntiles; k += RD_NT)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) a[c] += partial[((long long)m * ntiles + k) * 3 + c];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) s[c][t] = a[c];
+    __syncthreads();
+    for (int o = RD_NT / 2; o > 0; o >>= 1) {
+        if (t < o)
+#pragma unroll
+            for (int c = 0; c < 3; ++c) s[c][t] += s[c][t + o];
+        __syncthreads();
+    }
+    if (t < 3) grad[(long long)m * 3 + t] = s[t][0];
 }
 
 template <class T>
@@ -917,7 +944,7 @@ bool contract_dmma(int mode, int batch, int n, const double* W, long long ldw, l
         if ((*err = smem_optin(k_adjoint_contract_dmma<0, TNC>, SH::SMEM)) != cudaSuccess) return true;
         k_adjoint_contract_dmma<0, TNC><<<grid, SH::NT, SH::SMEM, st>>>(wmap, wmapj, n, alpha, astride, X, d, xstride,
                                                                         theta, tstride, partial, nullptr, 0, 0);
-        k_adjoint_reduce<<<batch, 32, 0, st>>>(ntiles, partial, grad);
+        k_adjoint_reduce<<<batch, RD_NT, 0, st>>>(ntiles, partial, grad);
         note_launches(2);
     } else {
         if ((*err = smem_optin(k_adjoint_contract_dmma<1, TNC>, SH::SMEM)) != cudaSuccess) return true;
@@ -927,6 +954,48 @@ bool contract_dmma(int mode, int batch, int n, const double* W, long long ldw, l
     }
     *err = cudaGetLastError();
     return true;
+}
+
+// FP32, one matrix: the same tiles by the packed FP32 tile product (sgemm.cuh), k over
+// [i0, n); W(k, i) counts for k >= i, what lies above W's diagonal is masked.
+__device__ int g_contract_status;
+template <int MODE, bool TMA>
+__global__ void __launch_bounds__(CT_NT, 1)
+    k_adjoint_contract_f32(const __grid_constant__ CUtensorMap map, int n, const float* __restrict__ W, long long ldw,
+                           const float* __restrict__ al, const float* __restrict__ x, int d,
+                           const double* __restrict__ th, double* __restrict__ partial, float* __restrict__ G,
+                           long long ldg)
+{
+    extern __shared__ __align__(128) unsigned char sg_raw[];
+    __shared__ double red[3][CT_NT / 32];
+    int ti, tj;
+    tile_of_lower(blockIdx.x, ti, tj);
+    const int i0 = ti * CT_TILE, j0 = tj * CT_TILE;
+    float acc[8][8];
+    sg::tile<true, true, TMA, sg::K_GE_ROW, sg::K_GE_ROW>(&map, &map, W, ldw, W, ldw, i0, j0, n, n, i0,
+                                                          (n - i0 + sg::KC - 1) / sg::KC, n, CT_TILE / sg::KC, 1 << 30,
+                                                          sg_raw, &g_contract_status, acc);
+    const int ty = sg::thread_row(), tx = sg::thread_col();
+    contract_epilogue<float, MODE>(n, acc, [&](int u) { return ty + 16 * u; }, [&](int v) { return tx + 16 * v; }, i0,
+                                   j0, al, x, d, th, red, partial + (long long)blockIdx.x * 3, G, ldg);
+}
+
+template <int MODE>
+int contract_f32(int ntiles, int n, const float* W, long long ldw, const float* alpha, const float* X, int d,
+                 const double* theta, double* partial, float* G, long long ldg, cudaStream_t st)
+{
+    constexpr size_t smem = sg::smem<true, true>();
+    CUtensorMap map{};
+    cudaError_t e;
+    if (sg::encode<true>(&map, W, n, ldw)) {
+        if ((e = smem_optin(k_adjoint_contract_f32<MODE, true>, smem)) != cudaSuccess) return (int)e;
+        k_adjoint_contract_f32<MODE, true><<<ntiles, CT_NT, smem, st>>>(map, n, W, ldw, alpha, X, d, theta, partial, G, ldg);
+    } else {
+        if ((e = smem_optin(k_adjoint_contract_f32<MODE, false>, smem)) != cudaSuccess) return (int)e;
+        k_adjoint_contract_f32<MODE, false><<<ntiles, CT_NT, smem, st>>>(map, n, W, ldw, alpha, X, d, theta, partial, G, ldg);
+    }
+    note_launches(1);
+    return (int)cudaGetLastError();
 }
 
 template <class T, bool DIRECT>
@@ -943,13 +1012,26 @@ int contract_t(int mode, int batch, int n, const void* W, long long ldw, long lo
     }
     const int nt = (n + CT_TILE - 1) / CT_TILE;
     const int ntiles = nt * (nt + 1) / 2;
+    if constexpr (std::is_same<T, float>::value && !DIRECT) {
+        if (batch == 1) {
+            const float *w = static_cast<const float*>(W), *al = static_cast<const float*>(alpha);
+            if (mode == 1)
+                return contract_f32<1>(ntiles, n, w, ldw, al, nullptr, 0, nullptr, nullptr, static_cast<float*>(G), ldg, st);
+            if (int e = contract_f32<0>(ntiles, n, w, ldw, al, static_cast<const float*>(X), d, theta, partial, nullptr,
+                                        0, st))
+                return e;
+            k_adjoint_reduce<<<batch, RD_NT, 0, st>>>(ntiles, partial, grad);
+            note_launches(1);
+            return (int)cudaGetLastError();
+        }
+    }
     dim3 grid(ntiles, batch);
     if (mode == 0) {
         k_adjoint_contract<T, 0, DIRECT><<<grid, CT_NT, 0, st>>>(n, static_cast<const T*>(W), ldw, wstride,
                                                          static_cast<const T*>(alpha), astride,
                                                          static_cast<const T*>(X), d, xstride, theta, tstride, partial,
                                                          nullptr, 0, 0);
-        k_adjoint_reduce<<<batch, 32, 0, st>>>(ntiles, partial, grad);
+        k_adjoint_reduce<<<batch, RD_NT, 0, st>>>(ntiles, partial, grad);
         note_launches(2);
     } else {
         k_adjoint_contract<T, 1, DIRECT><<<grid, CT_NT, 0, st>>>(n, static_cast<const T*>(W), ldw, wstride,

@@ -29,6 +29,15 @@ cudaError_t launch_trsm_panel_dmma(S* A, long long lda, long long astride, int b
 cudaError_t launch_syrk_batched(double* A, long long lda, long long astride, int batch, int k0, int nbk, int n,
                                 long long t0, int cols, const int* dinfo, cudaStream_t st);
 
+// The FP32 update of the region as trailing_update, nbk a multiple of 32 (sgemm.cu).
+template <bool UP>
+cudaError_t syrk_f32(float* A, long long lda, int k0, int nbk, int n, long long t0, int cols, const int* dinfo,
+                     cudaStream_t st);
+
+// W = L^-1 for one lower FP32 factor of any order; what W holds above its diagonal
+// afterwards is unspecified (sgemm.cu).
+cudaError_t trtri_large_f32(int n, const float* L, long long ldl, float* W, long long ldw, cudaStream_t st);
+
 template <class T, bool UP>
 cudaError_t trailing_update_simt(T* A, long long lda, int k0, int nbk, int n, long long t0, int cols,
                                  const int* dinfo, cudaStream_t st);

@@ -9,8 +9,9 @@
 //   2. L21 = A21 * L11^{-H}: real types on the FP64 tensor cores
 //      (k_trsm_panel_dmma, panel.cu); complex types by k_trsm_panel, warps own
 //      rows, lanes own columns, each solved entry broadcast with a warp shuffle;
-//   3. trailing update -- C -= L21 * L21^H on lower tiles (FP64 DMMA for double,
-//                        syrk.cu; register-tiled SIMT for the other types).
+//   3. trailing update -- C -= L21 * L21^H on lower tiles (FP64 DMMA for double and
+//                        lower complex double, syrk.cu; packed FP32 FMAs for float,
+//                        sgemm.cu; register-tiled SIMT for the rest).
 // Look-ahead: the update of block column k+1 plus the diagonal block and panel
 // of k+1 run on a high-priority internal stream while the update of the rest
 // of the trailing matrix runs on the caller's stream; events order the two so
@@ -149,7 +150,7 @@ long long trsm_grid(K* kernel, size_t smem, long long groups)
 }
 
 // ---------------------------------------------------------------------------
-// 3. generic trailing update (SIMT; every type).  64x64 tiles, 16-wide k
+// 3. generic trailing update (SIMT; the complex types).  64x64 tiles, 16-wide k
 //    chunks through shared memory, 4x4 per thread.  Region: rows [t0, n) and
 //    columns [t0, n) (cols == 0, lower triangle of tiles) or [t0, t0+cols).
 // ---------------------------------------------------------------------------
@@ -229,10 +230,6 @@ cudaError_t trailing_update_simt(T* A, long long lda, int k0, int nbk, int n, lo
 #define DDLAK_INST_SIMT(T, UP)                                                                                      \
     template cudaError_t trailing_update_simt<T, UP>(T*, long long, int, int, int, long long, int, const int*,     \
                                                      cudaStream_t);
-DDLAK_INST_SIMT(float, false)
-DDLAK_INST_SIMT(float, true)
-DDLAK_INST_SIMT(double, false)
-DDLAK_INST_SIMT(double, true)
 DDLAK_INST_SIMT(cf32, false)
 DDLAK_INST_SIMT(cf32, true)
 DDLAK_INST_SIMT(cf64, false)
@@ -384,13 +381,18 @@ static cudaError_t potrf_enqueue(T* A, long long lda, int n, int G, int* dinfo, 
 
 // Block columns per super-step.  A wide super-step reads and writes the trailing matrix
 // less often, but its left-looking updates (K up to 128 (G - 1) on one block column)
-// lie on the chain, which is all of the time at small orders.  FP64, ms with G = 1 / 2 /
-// 4 / 8: n = 2048 0.86 / 0.91 / 1.0 / 1.1; 5003 3.70 / 3.60 / 3.77 / 3.9; 8192 - / 8.99 /
-// 8.59 / 8.8; 16384 - / - / 52.4 / 50.1.
+// lie on the chain, which is all of the time at small orders.  ms with G = 1 / 2 / 4 / 8:
+//   d L  n = 2048 0.86 / 0.91 / 1.0 / 1.1    5003 3.70 / 3.60 / 3.77 / 3.9
+//        8192 - / 8.99 / 8.59 / 8.8          16384 - / - / 52.4 / 50.1
+//   s L  2048 1.56 / 1.57 / 1.74 / 2.15      6000 10.5 / 7.9 / 7.2 / 7.9   16384 184 / 101 / 63 / 49
+//   s U  2048 1.38 / 1.51 / 1.78 / 2.30      6000 6.2 / 6.0 / 6.8 / 8.6    16384 107 / 78 / 65 / 62
+//   c L  2048 3.20 / 3.32 / 3.64 / 4.30      6000 13.6 / 14.3 / 15.5 / 17.9  8192 25.9 / 25.7 / 27.4 / 30.8
+//   z L  2048 2.98 / 3.18 / 3.48 / 4.19      6000 16.5 / 15.4 / 16.1 / 18.4  8192 33.8 / 31.0 / 31.0 / 33.4
 static int potrf_group(char type, int n)
 {
-    if (type != 'd') return DDLAK_POTRF_GROUP;
-    return n < 3072 ? 1 : n < 6144 ? 2 : n < 12288 ? 4 : DDLAK_POTRF_GROUP;
+    if (n < 3072) return 1;
+    if (type == 'c') return n < 6144 ? 1 : n < 12288 ? 2 : DDLAK_POTRF_GROUP;
+    return n < 6144 ? 2 : n < 12288 ? 4 : DDLAK_POTRF_GROUP;
 }
 
 template <class T>

@@ -890,7 +890,8 @@ extern "C" int ddlak_forward_solve(char type, char uplo, char side, int n, int n
     }
 }
 
-// W = L^-1 for a lower factor: the fused forward substitution on the identity.
+// W = L^-1 for a lower factor: FP64 by the fused forward substitution on the identity,
+// FP32 by doubling (sgemm.cu).
 extern "C" int ddlak_trtri_blocked(char type, int n, const void* L, long long ldl, void* W, long long ldw, void* work,
                                    unsigned long long work_bytes, void* stream)
 {
@@ -906,8 +907,6 @@ extern "C" int ddlak_trtri_blocked(char type, int n, const void* L, long long ld
     if (type == 'd')
         return (int)potrs_launch<double, false, false, double, true>(
             static_cast<const double*>(L), ldl, static_cast<double*>(W), ldw, n, n, flags, ticket, status, st);
-    if (type == 's')
-        return (int)potrs_launch<float, false, false, float, true>(
-            static_cast<const float*>(L), ldl, static_cast<float*>(W), ldw, n, n, flags, ticket, status, st);
+    if (type == 's') return (int)trtri_large_f32(n, static_cast<const float*>(L), ldl, static_cast<float*>(W), ldw, st);
     return (int)cudaErrorInvalidValue;
 }

@@ -4,7 +4,8 @@
 // (src/Cholesky/potrf.cpp:111) and, on multi-rank grids, to herk/gemm
 // (src/Cholesky/ppotrf.cpp:212-238).  For double it runs on the FP64 tensor
 // cores: mma.sync m16n8k4 f64 (DMMA).  Complex double (lower) runs as two real
-// DMMA products per fragment; the other types use the SIMT kernel in potrf.cu.
+// DMMA products per fragment; float runs on packed FP32 FMAs (sgemm.cu), the other
+// complex forms on the SIMT kernel in potrf.cu.
 #include <cuda.h>
 
 #include <type_traits>
@@ -510,11 +511,13 @@ cudaError_t trailing_update(T* A, long long lda, int k0, int nbk, int n, long lo
     if constexpr (std::is_same<T, double>::value) {
         return syrk_dmma<UP, false>(A, lda, 0, 1, k0, nbk, n, t0, cols, dinfo, st);
     }
+    if constexpr (std::is_same<T, float>::value) return syrk_f32<UP>(A, lda, k0, nbk, n, t0, cols, dinfo, st);
     if constexpr (std::is_same<T, cf64>::value && !UP) {
         cudaError_t e = cudaSuccess;
         if (launch_zmma_tma(A, lda, k0, nbk, n, t0, cols, dinfo, st, &e)) return e;
     }
-    return trailing_update_simt<T, UP>(A, lda, k0, nbk, n, t0, cols, dinfo, st);
+    if constexpr (Traits<T>::cplx) return trailing_update_simt<T, UP>(A, lda, k0, nbk, n, t0, cols, dinfo, st);
+    return cudaErrorInvalidValue;
 }
 
 #define DDLAK_INST_TU(T, UP)                                                                                        \
