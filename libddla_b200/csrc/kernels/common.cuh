@@ -105,6 +105,17 @@ __device__ __forceinline__ void lview_st(T* A, long long lda, long long i, long 
     else A[i + j * lda] = v;
 }
 
+// 1/sqrt(d) for a positive normal d: the hardware's approximation (about 20 bits)
+// and one step of Householder's third-order iteration for y^-2 = d,
+// y <- y + y (e/2 + 3 e^2/8), e = 1 - d y^2, which cubes the relative error.
+__device__ __forceinline__ double rsqrt_pivot(double d)
+{
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
+    const double e = fma(-d * y, y, 1.0);
+    return fma(fma(0.375, e, 0.5), y * e, y);
+}
+
 // Status words written by kernels that wait on other CTAs.  A wait gives up
 // after a clock budget and records one of these instead of spinning forever.
 enum : int {

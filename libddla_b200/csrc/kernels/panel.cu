@@ -21,6 +21,7 @@
 #include "common.cuh"
 #include "ddla_kernels_internal.h"
 #include "profile.h"
+#include "tile8.cuh"
 
 namespace ddlak {
 
@@ -35,17 +36,6 @@ __device__ __forceinline__ void dmma4(double (&d)[4], const double (&c)[4], doub
     asm volatile("mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%7,%8,%9,%10};"
                  : "=d"(d[0]), "=d"(d[1]), "=d"(d[2]), "=d"(d[3])
                  : "d"(a_up), "d"(a_lo), "d"(b), "d"(c[0]), "d"(c[1]), "d"(c[2]), "d"(c[3]));
-}
-
-// 1/sqrt(d) for a positive normal d: the hardware's approximation (about 20 bits)
-// and one step of Householder's third-order iteration for y^-2 = d,
-// y <- y + y (e/2 + 3 e^2/8), e = 1 - d y^2, which cubes the relative error.
-__device__ __forceinline__ double rsqrt_pivot(double d)
-{
-    double y;
-    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
-    const double e = fma(-d * y, y, 1.0);
-    return fma(fma(0.375, e, 0.5), y * e, y);
 }
 
 template <bool UP>
@@ -90,6 +80,7 @@ __global__ void __launch_bounds__(DG_THREADS, 1) k_potrf_diag_dmma(S* __restrict
 {
     __shared__ __align__(16) double T[64];        // the diagonal tile, row-major
     __shared__ __align__(16) double Inv[64];      // its inverse, row-major
+    __shared__ __align__(16) double Lt[64];       // its factor, row-major (warp 0's own)
     __shared__ __align__(16) double Xs[PN_NB * 8];  // the step's X, row-major
     __shared__ int s_fail;                        // 0, or 1 + the failed column of the current tile
     A += (long long)blockIdx.x * astride;  // blockIdx.x: the matrix of a batch
@@ -103,54 +94,16 @@ __global__ void __launch_bounds__(DG_THREADS, 1) k_potrf_diag_dmma(S* __restrict
     if (warp == 0) {
         for (int j = 0; j < steps; ++j) {
             bar_sync<1, 64>();  // T is in
-            double a[8][8];
-#pragma unroll
-            for (int r = 0; r < 8; ++r)
-#pragma unroll
-                for (int h = 0; h <= r / 2; ++h) {
-                    const double2 v = *reinterpret_cast<const double2*>(&T[r * 8 + 2 * h]);
-                    a[r][2 * h] = v.x;
-                    a[r][2 * h + 1] = v.y;
-                }
-            double y[8];
-#pragma unroll
-            for (int i = 0; i < 8; ++i) y[i] = (lane & 7) == i ? 1.0 : 0.0;
-            int good = 8;  // final columns
-#pragma unroll
-            for (int k = 0; k < 8; ++k) {
-                const double d = a[k][k];
-                if (good == 8 && !(d > 0.0)) good = k;
-                const bool live = good == 8;
-                const double r = live ? rsqrt_pivot(d) : 0.0;
-#pragma unroll
-                for (int i = k + 1; i < 8; ++i) {
-                    const double l = a[i][k] * r;
-#pragma unroll
-                    for (int m = k + 1; m < i; ++m) a[i][m] = fma(-l, a[m][k], a[i][m]);
-                    a[i][i] = fma(-l, l, a[i][i]);
-                    if (live) a[i][k] = l;
-                }
-                // column k of L is now in a[.][k] (rows m < i above read the scaled entries)
-                const double s = d * r;
-                if (live) a[k][k] = fma(0.5 * r, fma(-s, s, d), s);
-                y[k] *= r;
-#pragma unroll
-                for (int i = k + 1; i < 8; ++i)
-                    if (live) y[i] = fma(-a[i][k], y[k], y[i]);
-            }
-            if (lane < 8) {
-#pragma unroll
-                for (int i = 0; i < 8; ++i) Inv[i * 8 + lane] = y[i];
-            }
+            const int good = factor_tile8(T, Inv, Lt, nullptr, 8, lane);
             if (lane == 0) s_fail = good == 8 ? 0 : good + 1;
             bar_sync<2, DG_THREADS>();
-            // the tile itself
+            // the tile itself, two entries a lane
 #pragma unroll
-            for (int r = 0; r < 8; ++r)
-#pragma unroll
-                for (int c = 0; c <= r; ++c)
-                    if (lane == ((r * 8 + c) & 31) && 8 * j + r < nbk)
-                        Ab[lpos<UP>(lda, 8 * j + r, 8 * j + c)] = (S)a[r][c];
+            for (int x = 0; x < 2; ++x) {
+                const int e = lane + 32 * x, r = UP ? e >> 3 : e & 7, c = UP ? e & 7 : e >> 3;
+                if (c <= r && 8 * j + r < nbk) Ab[lpos<UP>(lda, 8 * j + r, 8 * j + c)] = (S)Lt[r * 8 + c];
+            }
+            __syncwarp();
             if (good < 8) {
                 if (lane == 0) *info = k0 + 8 * j + good + 1;
                 return;

@@ -1,0 +1,79 @@
+// Cholesky of one 8 x 8 tile with its inverse, by one warp (the pivot chain of panel.cu and
+// vbatched.cu).
+#pragma once
+#include "common.cuh"
+
+namespace ddlak {
+
+// T: the tile in shared memory, row-major, lower part.  Its first kv columns are factored,
+// redundantly in every lane (a column costs one reciprocal square root, a multiply and a
+// multiply-add, no shuffles; lane c carries column c of the inverse along): L into Lt
+// (row-major; the columns before a failed one final, that one with the values updated by
+// them), the inverse into Inv (row-major; its rows from a failed column on are zero), 1 / l_kk
+// into rinv[k] when given.  Returns the number of factored columns: kv, or the index of the
+// first pivot that is not positive.  Rows from kv on are solved against the columns before kv
+// like any row below; their own columns are decoupled by a huge diagonal.
+// Everything is straight-line code on values all lanes hold, stores included (every lane
+// stores the same word): predicating the 36 stores of L on a lane each made the tile take
+// 7900 clocks instead of 1000.
+__device__ __forceinline__ int factor_tile8(const double* T, double* Inv, double* Lt, double* rinv, int kv, int lane)
+{
+    double a[8][8], y[8];
+#pragma unroll
+    for (int r = 0; r < 8; ++r)
+#pragma unroll
+        for (int h = 0; h <= r / 2; ++h) {
+            const double2 v = *reinterpret_cast<const double2*>(&T[r * 8 + 2 * h]);
+            a[r][2 * h] = v.x;
+            a[r][2 * h + 1] = v.y;
+        }
+#pragma unroll
+    for (int r = 1; r < 8; ++r)
+        if (r >= kv) {  // uniform
+#pragma unroll
+            for (int c = 0; c < r; ++c)
+                if (c >= kv) a[r][c] = 0.0;
+            a[r][r] = 1e300;
+        }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) y[i] = (lane & 7) == i ? 1.0 : 0.0;
+    int good = 8;
+    double rk = 0.0;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        const double d = a[k][k];
+        if (good == 8 && !(d > 0.0)) good = k;
+        const bool live = good == 8;
+        const double rs = rsqrt_pivot(d);
+        const double r = live ? rs : 0.0;
+        rk = lane == k ? r : rk;
+#pragma unroll
+        for (int i = k + 1; i < 8; ++i) {
+            const double l = a[i][k] * r;
+#pragma unroll
+            for (int m = k + 1; m < i; ++m) a[i][m] = fma(-l, a[m][k], a[i][m]);
+            a[i][i] = fma(-l, l, a[i][i]);
+            a[i][k] = live ? l : a[i][k];
+        }
+        const double s = d * r;
+        a[k][k] = live ? fma(0.5 * r, fma(-s, s, d), s) : d;
+        y[k] *= r;
+#pragma unroll
+        for (int i = k + 1; i < 8; ++i) y[i] = fma(live ? -a[i][k] : 0.0, y[k], y[i]);
+    }
+    good = good < kv ? good : kv;
+    if (lane < 8) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) Inv[i * 8 + lane] = y[i];
+        if (rinv != nullptr && lane < good) rinv[lane] = rk;
+    }
+#pragma unroll
+    for (int r = 0; r < 8; ++r)
+#pragma unroll
+        for (int h = 0; h <= r / 2; ++h)
+            *reinterpret_cast<double2*>(&Lt[r * 8 + 2 * h]) = make_double2(a[r][2 * h], 2 * h + 1 <= r ? a[r][2 * h + 1] : 0.0);
+    __syncwarp();
+    return good;
+}
+
+}  // namespace ddlak
