@@ -324,10 +324,10 @@ __global__ void __launch_bounds__(NT) k_potrs_fused(const T* __restrict__ A, lon
 //   * One thread polls the flag of the block needed; every warp reads that block's
 //     solution straight into its operand fragments; the next one is fetched under
 //     the current product when its flag is already up.
-// What bounds it: the chain of n / 64 links per direction.  Measured (factor and flags
-// in place, one call): n = 2048, 16 right-hand sides 345 against 556 us for the
-// substitution form, n = 5003, 3 of them 0.88 against 1.38 ms; n = 16384, 64 of them
-// 6.6 ms either way.
+// What bounds it: the chain of n / 64 links per direction.  Measured (one call, factor
+// and flags in place) against the substitution form: n = 2048, 16 right-hand sides 240
+// against 556 us; n = 5003, 3 of them 0.56 against 1.38 ms; n = 16384, 64 of them 4.8
+// against 6.6 ms.
 // ---------------------------------------------------------------------------
 constexpr int PD_LD = RB + 4;  // 4 mod 16 doubles: conflict-free fragment reads either way round
 constexpr int PD_LDX = RC + 4;
@@ -341,7 +341,7 @@ __host__ __device__ constexpr size_t potrs_dmma_smem()
 
 __device__ __forceinline__ void pd_mma(double (&d)[4], double a_up, double a_lo, double b)
 {
-    asm volatile("mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};"
+    asm("mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};"
                  : "+d"(d[0]), "+d"(d[1]), "+d"(d[2]), "+d"(d[3])
                  : "d"(a_up), "d"(a_lo), "d"(b));
 }
@@ -508,8 +508,13 @@ __global__ void __launch_bounds__(NT, 2) k_potrs_dmma(const TL* __restrict__ A, 
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
             const long long i = i0 + row + 8 * h, r = rc + 2 * q + e;
-            if (ID) acc[2 * h + e] = i == r && i < n ? 1.0 : 0.0;
-            else acc[2 * h + e] = row + 8 * h < nrows && r < nrhs ? (double)x_ld_cg<TX, BT>(B, ldb, i, r) : 0.0;
+            if (ID) {
+                acc[2 * h + e] = i == r && i < n ? 1.0 : 0.0;
+            } else {
+                const bool in = row + 8 * h < nrows && r < nrhs;
+                const double v = (double)x_ld_cg<TX, BT>(B, ldb, in ? i : 0, in ? r : 0);
+                acc[2 * h + e] = in ? v : 0.0;
+            }
         }
     double xr[RB / 4];  // operand fragments of the other block's solution: X(k = 4 m + q, r = g), negated
     bool pre = false;
@@ -517,8 +522,12 @@ __global__ void __launch_bounds__(NT, 2) k_potrs_dmma(const TL* __restrict__ A, 
         const long long j0 = (long long)j * RB;
 #pragma unroll
         for (int m = 0; m < RB / 4; ++m) {
+            // unconditional (of B(0, 0) where there is nothing to load): as branches the 16 loads
+            // took their latencies one after the other, 5000 of a link's 11000 clocks
             const long long k = j0 + 4 * m + q;
-            xr[m] = k < n && rc + g < nrhs ? -(double)x_ld_cg<TX, BT>(B, ldb, k, rc + g) : 0.0;
+            const bool in = k < n && rc + g < nrhs;
+            const double v = (double)x_ld_cg<TX, BT>(B, ldb, in ? k : 0, in ? rc + g : 0);
+            xr[m] = in ? -v : 0.0;
         }
     };
     for (int v = 0; v < nvisit; ++v) {
