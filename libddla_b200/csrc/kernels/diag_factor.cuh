@@ -41,22 +41,6 @@ __device__ __forceinline__ T shfl(T v, int src)
 
 namespace diagf {
 
-// 1/d for the pivots on the column chain: the hardware's approximate reciprocal
-// (rcp.approx.ftz.f64, about single precision) refined by two Newton-Raphson
-// steps r <- r + r (1 - d r), each of which squares the relative error, so the
-// result is within an ulp or two of 1/d for the positive normal pivots this is
-// used on (a non-positive pivot stops the factorization before its reciprocal
-// is used).  Cheaper on the chain than the correctly rounded division.
-__device__ __forceinline__ double recip_pivot(double d)
-{
-    double r;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
-    double e = fma(-d, r, 1.0);
-    r = fma(r, e, r);
-    e = fma(-d, r, 1.0);
-    return fma(r, e, r);
-}
-__device__ __forceinline__ float recip_pivot(float d) { return 1.0f / d; }
 
 constexpr int PW = 32;    // panel width
 constexpr int MAXN = 128;  // largest block

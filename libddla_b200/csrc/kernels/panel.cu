@@ -30,12 +30,31 @@ namespace {
 constexpr int PN_NB = 128;           // block order
 constexpr int PN_TILES = PN_NB / 8;  // 8-column steps
 
-// d = c + a b, fragments as above (u: row g, v: row g + 8, columns 2q + e)
+// d = c + a b, fragments as above (u: row g, v: row g + 8, columns 2q + e).  Not volatile:
+// the two products of a tile depend on each other, and only if the compiler may put other
+// tiles' between them is their latency (25 clocks) hidden.
 __device__ __forceinline__ void dmma4(double (&d)[4], const double (&c)[4], double a_up, double a_lo, double b)
 {
-    asm volatile("mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%7,%8,%9,%10};"
+    asm("mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%7,%8,%9,%10};"
                  : "=d"(d[0]), "=d"(d[1]), "=d"(d[2]), "=d"(d[3])
                  : "d"(a_up), "d"(a_lo), "d"(b), "d"(c[0]), "d"(c[1]), "d"(c[2]), "d"(c[3]));
+}
+
+// C_(l-1) = C_l - X B_l^T for the strip's tiles L0 <= l < L0 + G, as straight-line code: all the
+// operand loads, then the first products, then the second ones, so that neither the loads'
+// nor the products' latency is exposed (with a branch per tile a product took 59 clocks).
+// tile(l) gives this lane's operand pair of tile l; it is called past the last tile too.
+template <int L0, int G, class Tile>
+__device__ __forceinline__ void strip_update(double (&C)[PN_TILES][4], const double (&X)[4], Tile tile)
+{
+    double2 b[G];
+    double Y[G][4];
+#pragma unroll
+    for (int i = 0; i < G; ++i) b[i] = tile(L0 + i);
+#pragma unroll
+    for (int i = 0; i < G; ++i) dmma4(Y[i], C[L0 + i], -X[0], -X[2], b[i].x);
+#pragma unroll
+    for (int i = 0; i < G; ++i) dmma4(C[L0 + i - 1], Y[i], -X[1], -X[3], b[i].y);
 }
 
 template <bool UP>
@@ -71,8 +90,9 @@ __device__ __forceinline__ void bar_arrive()
 // fewest tiles, so the chain does not queue behind the strips' DMMAs.
 // info as LAPACK ?potrf: the first pivot that is not positive; the columns
 // before it are final, it keeps its updated value.
-// What bounds it: the chain of 128 dependent pivots.  Measured on one B200: 19.6 us a
-// block, against 36.2 us for 32-column panels with one warp's shared-memory column chain.
+// What bounds it: the chain of 128 dependent pivots, 16 steps of some 1900 clocks (the tile
+// 1150, the hand-overs and the next tile's update the rest).  Measured on one B200: 16 us a
+// block, against 36 us for 32-column panels with one warp's shared-memory column chain.
 // ---------------------------------------------------------------------------
 template <class S, bool UP>
 __global__ void __launch_bounds__(DG_THREADS, 1) k_potrf_diag_dmma(S* __restrict__ A, long long lda, long long astride,
@@ -128,6 +148,19 @@ __global__ void __launch_bounds__(DG_THREADS, 1) k_potrf_diag_dmma(S* __restrict
                 if (c <= r && r < nbk) C[l][2 * h + e] = (double)Ab[lpos<UP>(lda, r, c)];
             }
     }
+    // rows below step j's diagonal tile, the tile's first `good` columns
+    auto store = [&](int j, const double (&X)[4], int good) {
+        if (2 * w + 1 < j) return;
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int r = h ? r_lo : r_up, c = 2 * q + e;
+                if (r >= 8 * (j + 1) && r < nbk && c < good) Ab[lpos<UP>(lda, r, 8 * j + c)] = (S)X[2 * h + e];
+            }
+    };
+    double X[4] = {0.0, 0.0, 0.0, 0.0};
+    int fail = 0;
 #pragma unroll 1
     for (int j = 0; j < steps; ++j) {
         const int cnt = 2 * w + 1 - j;  // tiles of this strip after tile j
@@ -136,9 +169,9 @@ __global__ void __launch_bounds__(DG_THREADS, 1) k_potrf_diag_dmma(S* __restrict
             else *reinterpret_cast<double2*>(&T[g * 8 + 2 * q]) = make_double2(C[0][0], C[0][1]);
             bar_arrive<1, 64>();
         }
-        bar_sync<2, DG_THREADS>();  // Inv and s_fail are in
-        const int fail = s_fail;
-        double X[4] = {0.0, 0.0, 0.0, 0.0};
+        if (j > 0) store(j - 1, X, 8);  // once the tile is handed over: off the chain
+        bar_sync<2, DG_THREADS>();      // Inv and s_fail are in
+        fail = s_fail;
         if (cnt >= 0) {
             const double2 b = *reinterpret_cast<const double2*>(&Inv[g * 8 + 2 * q]);
             const double z[4] = {0.0, 0.0, 0.0, 0.0};
@@ -149,30 +182,21 @@ __global__ void __launch_bounds__(DG_THREADS, 1) k_potrf_diag_dmma(S* __restrict
             *reinterpret_cast<double2*>(&Xs[r_lo * 8 + 2 * q]) = make_double2(X[2], X[3]);
         }
         bar_sync<3, 32 * DG_WORKERS>();
-        if (!fail) {
-#pragma unroll
-            for (int l = 1; l < PN_TILES; ++l) {
-                if (l > cnt) break;
-                const double2 b = *reinterpret_cast<const double2*>(&Xs[(8 * (j + l) + g) * 8 + 2 * q]);
-                double Y[4];
-                dmma4(Y, C[l], -X[0], -X[2], b.x);
-                dmma4(C[l - 1], Y, -X[1], -X[3], b.y);
-            }
+        if (fail) {  // uniform over the workers
+            store(j, X, fail - 1);
+            return;
         }
-        // rows below the diagonal tile, the tile's final columns
-        if (cnt >= 0) {
-            const int good = fail ? fail - 1 : 8;
+        // (a branch per tile: the owner of the next diagonal tile, on the chain, has one or two)
 #pragma unroll
-            for (int h = 0; h < 2; ++h)
-#pragma unroll
-                for (int e = 0; e < 2; ++e) {
-                    const int r = h ? r_lo : r_up, c = 2 * q + e;
-                    if (r >= 8 * (j + 1) && r < nbk && c < good)
-                        Ab[lpos<UP>(lda, r, 8 * j + c)] = (S)X[2 * h + e];
-                }
+        for (int l = 1; l < PN_TILES; ++l) {
+            if (l > cnt) break;
+            const double2 b = *reinterpret_cast<const double2*>(&Xs[(8 * (j + l) + g) * 8 + 2 * q]);
+            double Y[4];
+            dmma4(Y, C[l], -X[0], -X[2], b.x);
+            dmma4(C[l - 1], Y, -X[1], -X[3], b.y);
         }
-        if (fail) return;  // uniform over the workers
     }
+    store(steps - 1, X, 8);
 }
 
 template <class S, bool UP>
@@ -190,10 +214,10 @@ cudaError_t launch_potrf_diag(S* A, long long lda, long long astride, int batch,
 // 16-byte units of a row rotated by half the row index so that fragment loads
 // and the column-wise fill are spread over the banks), the diagonal tiles'
 // inverses formed by 128 threads (one column each) on the way.
-// What bounds it: 272 DMMAs per strip (32 clocks each on a scheduler's FP64
-// pipe, 4.6 us), after L11's load.  Measured: 19.8 us for the panels of n = 2048, against
-// 33 us for one thread per row; 42.7 against 54.7 us on average over n = 16384 (beside
-// the trailing update).  No alignment is asked of A, so there is one form for all.
+// What bounds it: 272 DMMAs per strip (34 clocks each on a scheduler's FP64 pipe, 4.9 us),
+// after L11's load and the inverses.  Measured: 13 us for the panels of n = 2048 (load 2.6,
+// inverses 0.7, steps 9.4), against 33 us for one thread per row.  No alignment is asked of
+// A, so there is one form for all.
 // ---------------------------------------------------------------------------
 namespace {
 constexpr int TR_NT = 128, TR_ROWS = 64;
@@ -210,6 +234,7 @@ __global__ void __launch_bounds__(TR_NT) k_trsm_panel_dmma(S* __restrict__ A, lo
                                                            int nbk, int n, const int* __restrict__ info)
 {
     extern __shared__ __align__(16) double tr_smem[];
+    __shared__ double Rp[PN_NB];
     double* Lt = tr_smem;
     double* Inv = tr_smem + TR_LTILES * 64;  // row-major 8 x 8 tiles
     A += (long long)blockIdx.y * astride;    // blockIdx.y: the matrix of a batch
@@ -218,59 +243,86 @@ __global__ void __launch_bounds__(TR_NT) k_trsm_panel_dmma(S* __restrict__ A, lo
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
     const int g = lane >> 2, q = lane & 3;
     const S* Ad = A + lpos<UP>(lda, k0, k0);
-    // thread t fills row t ('L': coalesced over rows) or column t ('U': over columns) of L11
-    if constexpr (std::is_same<S, double>::value) {
-#pragma unroll 8
-        for (int o = 0; o < PN_NB; ++o) {
-            const int r = UP ? o : t, c = UP ? t : o;
-            if ((c >> 3) > (r >> 3)) continue;
-            const bool in = c <= r && r < nbk;
-            cp_async_elem<8>(&Lt[tr_tile(r >> 3, c >> 3) + tr_elem(r & 7, c & 7)], in ? Ad + lpos<UP>(lda, r, c) : Ad,
-                             in);
-        }
-        cp_group_commit();
-    } else {
-        for (int o0 = 0; o0 < PN_NB; o0 += 16) {
-            S v[16];
+    // L11's tiles: a thread takes every other tile of line t and the others of line 127 - t ('L': a
+    // line is a row, its tiles to the left of the diagonal; 'U': a column, its tiles below), so
+    // that all threads copy about as much; consecutive threads on consecutive words
+    auto fill = [&](int line, int par) {
+        const int lt = line >> 3, li = line & 7;
+        int off[8];  // word of the line's m-th entry in a tile
 #pragma unroll
-            for (int u = 0; u < 16; ++u) {
-                const int r = UP ? o0 + u : t, c = UP ? t : o0 + u;
-                v[u] = c <= r && r < nbk ? Ad[lpos<UP>(lda, r, c)] : S(0);
-            }
+        for (int m = 0; m < 8; ++m) off[m] = UP ? tr_elem(m, li) : tr_elem(li, m);
+        for (int o = (UP ? lt : 0) + par; o < (UP ? PN_TILES : lt + 1); o += 2) {
+            double* dst = Lt + (UP ? tr_tile(o, lt) : tr_tile(lt, o));
+            const S* src = Ad + lpos<UP>(lda, UP ? 8 * o : line, UP ? line : 8 * o);
+            const long long step = lda;  // the next entry of the line
+            S v[8];
 #pragma unroll
-            for (int u = 0; u < 16; ++u) {
-                const int r = UP ? o0 + u : t, c = UP ? t : o0 + u;
-                if ((c >> 3) <= (r >> 3)) Lt[tr_tile(r >> 3, c >> 3) + tr_elem(r & 7, c & 7)] = (double)v[u];
+            for (int m = 0; m < 8; ++m) {
+                const int r = UP ? 8 * o + m : line, c = UP ? line : 8 * o + m;
+                const bool in = c <= r && r < nbk;
+                if constexpr (std::is_same<S, double>::value) {
+                    cp_async_elem<8>(dst + off[m], in ? src + m * step : Ad, in);
+                } else {
+                    v[m] = *(in ? src + m * step : Ad);
+                    if (!in) v[m] = S(0);
+                }
+            }
+            if constexpr (!std::is_same<S, double>::value) {
+#pragma unroll
+                for (int m = 0; m < 8; ++m) dst[off[m]] = (double)v[m];
             }
         }
-    }
+    };
+    fill(t, 0);
+    fill(PN_NB - 1 - t, 1);
+    if constexpr (std::is_same<S, double>::value) cp_group_commit();
     // this warp's strip (its loads overlap the fill above)
     const long long row0 = (long long)k0 + nbk + (long long)blockIdx.x * TR_ROWS + warp * 16;
     const long long r_up = row0 + g, r_lo = r_up + 8;
     double C[PN_TILES][4];
+    if (nbk == PN_NB && row0 + 16 <= n) {  // whole strip: plain loads, in flight until the loop needs them
+        const S* in = A + lpos<UP>(lda, r_up, k0 + 2 * q);
+        const long long e_col = UP ? 1 : lda, e_row = UP ? 8 * lda : 8;
 #pragma unroll
-    for (int l = 0; l < PN_TILES; ++l)
+        for (int l = 0; l < PN_TILES; ++l)
 #pragma unroll
-        for (int h = 0; h < 2; ++h)
+            for (int h = 0; h < 2; ++h)
 #pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                const long long r = h ? r_lo : r_up;
-                const int c = 8 * l + 2 * q + e;
-                C[l][2 * h + e] = r < n && c < nbk ? (double)A[lpos<UP>(lda, r, k0 + c)] : 0.0;
-            }
+                for (int e = 0; e < 2; ++e) C[l][2 * h + e] = (double)in[(8 * l + e) * e_col + h * e_row];
+    } else {
+#pragma unroll
+        for (int l = 0; l < PN_TILES; ++l)
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const long long r = h ? r_lo : r_up;
+                    const int c = 8 * l + 2 * q + e;
+                    C[l][2 * h + e] = r < n && c < nbk ? (double)A[lpos<UP>(lda, r, k0 + c)] : 0.0;
+                }
+    }
     if constexpr (std::is_same<S, double>::value) cp_group_wait<0>();
     __syncthreads();
+    // the reciprocal pivots, one a thread (rows at or past nbk: the identity)
+    Rp[t] = t < nbk ? recip_pivot(Lt[tr_tile(t >> 3, t >> 3) + tr_elem(t & 7, t & 7)]) : 1.0;
+    __syncthreads();
     {
-        // column c of tile b's inverse: L y = e_c (rows at or past nbk: the identity)
+        // column c of tile b's inverse: L y = e_c
         const int b = t >> 3, c = t & 7;
         const double* tile = Lt + tr_tile(b, b);
-        double y[8];
+        double l[8][8], y[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+#pragma unroll
+            for (int k = 0; k < i; ++k) l[i][k] = tile[tr_elem(i, k)];
+            l[i][i] = Rp[8 * b + i];
+        }
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
             double s = i == c ? 1.0 : 0.0;
 #pragma unroll
-            for (int k = 0; k < i; ++k) s = fma(-tile[tr_elem(i, k)], y[k], s);
-            y[i] = 8 * b + i < nbk ? s / tile[tr_elem(i, i)] : s;
+            for (int k = 0; k < i; ++k) s = fma(-l[i][k], y[k], s);
+            y[i] = s * l[i][i];
         }
 #pragma unroll
         for (int i = 0; i < 8; ++i) Inv[b * 64 + i * 8 + c] = y[i];
@@ -279,6 +331,8 @@ __global__ void __launch_bounds__(TR_NT) k_trsm_panel_dmma(S* __restrict__ A, lo
     if (row0 >= n) return;
     const int steps = (nbk + 7) >> 3;
     const int unit = ((q ^ (g >> 1)) << 1) + g * 8;
+    S* out = A + lpos<UP>(lda, r_up, k0 + 2 * q);  // this lane's entries of the step's columns
+    const long long e_col = UP ? 1 : lda, e_row = UP ? 8 * lda : 8, e_step = UP ? 8 : 8 * lda;
 #pragma unroll 1
     for (int j = 0; j < steps; ++j) {
         double X[4];
@@ -289,23 +343,22 @@ __global__ void __launch_bounds__(TR_NT) k_trsm_panel_dmma(S* __restrict__ A, lo
             dmma4(Y, z, C[0][0], C[0][2], b.x);
             dmma4(X, Y, C[0][1], C[0][3], b.y);
         }
-#pragma unroll
-        for (int h = 0; h < 2; ++h)
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                const long long r = h ? r_lo : r_up;
-                const int c = 8 * j + 2 * q + e;
-                if (r < n && c < nbk) A[lpos<UP>(lda, r, k0 + c)] = (S)X[2 * h + e];
-            }
         const int cnt = steps - 1 - j;
+        auto tile = [&](int l) {
+            const int r = j + l < PN_TILES ? j + l : PN_TILES - 1;
+            return *reinterpret_cast<const double2*>(&Lt[tr_tile(r, j) + unit]);
+        };
 #pragma unroll
-        for (int l = 1; l < PN_TILES; ++l) {
-            if (l > cnt) break;
-            const double2 b = *reinterpret_cast<const double2*>(&Lt[tr_tile(j + l, j) + unit]);
-            double Y[4];
-            dmma4(Y, C[l], -X[0], -X[2], b.x);
-            dmma4(C[l - 1], Y, -X[1], -X[3], b.y);
+        for (int e = 0; e < 2; ++e) {
+            if (8 * j + 2 * q + e < nbk) {
+                if (r_up < n) out[e * e_col] = (S)X[e];
+                if (r_lo < n) out[e * e_col + e_row] = (S)X[2 + e];
+            }
         }
+        out += e_step;
+        if (cnt >= 1) strip_update<1, 5>(C, X, tile);
+        if (cnt >= 6) strip_update<6, 5>(C, X, tile);
+        if (cnt >= 11) strip_update<11, 5>(C, X, tile);
     }
 }
 
