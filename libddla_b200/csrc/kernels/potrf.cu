@@ -446,22 +446,25 @@ __global__ void __launch_bounds__(PB_NT) k_potrs_batched_f64(int n, const double
         __syncthreads();
         if (warp == 0) {
             double xi = lane < w ? x[b0 + lane] : 0.0;
-            for (int j = 0; j < w; ++j) {
-                if (lane == j) {
-                    const double d = blk[j][j];
-                    xi = xi / d;
-                    ld += log(d);
-                }
+            const double dl = lane < w ? blk[lane][lane] : 1.0, ri = 1.0 / dl;
+            ld += log(dl);
+#pragma unroll 8
+            for (int j = 0; j < 32; ++j) {  // columns at or past w are zero
+                if (lane == j) xi *= ri;
                 const double xj = __shfl_sync(0xffffffffu, xi, j);
-                if (lane > j && lane < w) xi = fma(-blk[lane][j], xj, xi);
+                if (lane > j) xi = fma(-blk[lane][j], xj, xi);
             }
             if (lane < w) x[b0 + lane] = xi;
         }
         __syncthreads();
-        for (int r = b0 + 32 + t; r < n; r += PB_NT) {
+        for (int r = b0 + 32 + t; r < n; r += PB_NT) {  // only below a full block (w = 32)
             double acc = x[r];
             const double* lr = L + r + (long long)b0 * lda;
-            for (int j = 0; j < w; ++j) acc = fma(-lr[(long long)j * lda], x[b0 + j], acc);
+            double l[32];
+#pragma unroll
+            for (int j = 0; j < 32; ++j) l[j] = lr[(long long)j * lda];
+#pragma unroll
+            for (int j = 0; j < 32; ++j) acc = fma(-l[j], x[b0 + j], acc);
             x[r] = acc;
         }
         __syncthreads();
@@ -473,14 +476,26 @@ __global__ void __launch_bounds__(PB_NT) k_potrs_batched_f64(int n, const double
     }
     for (int b0 = ((n - 1) / 32) * 32; b0 >= 0; b0 -= 32) {
         const int w = n - b0 < 32 ? n - b0 : 32;
-        // x_i -= sum_{r >= b0 + 32} l(r, b0 + i) x_r for the block's columns i
-        for (int i = warp; i < w; i += PB_NT / 32) {
-            const double* lc = L + (long long)(b0 + i) * lda;
-            double acc = 0.0;
-            for (int r = b0 + 32 + lane; r < n; r += 32) acc = fma(lc[r], x[r], acc);
+        // x_i -= sum_{r >= b0 + 32} l(r, b0 + i) x_r for the block's columns i (w = 32 when there is such r)
+        if (b0 + 32 < n) {
+            constexpr int CW = 32 / (PB_NT / 32);
+            const double* lc = L + (long long)(b0 + CW * warp) * lda;
+            double acc[CW];
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-            if (lane == 0) x[b0 + i] -= acc;
+            for (int c = 0; c < CW; ++c) acc[c] = 0.0;
+#pragma unroll 4
+            for (int r = b0 + 32 + lane; r < n; r += 32) {
+                const double xr = x[r];
+#pragma unroll
+                for (int c = 0; c < CW; ++c) acc[c] = fma(lc[r + c * lda], xr, acc[c]);
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+                for (int c = 0; c < CW; ++c) acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], o);
+            if (lane == 0)
+#pragma unroll
+                for (int c = 0; c < CW; ++c) x[b0 + CW * warp + c] -= acc[c];
         }
         for (int e = t; e < 32 * 32; e += PB_NT) {  // the block itself, for the transposed solve
             const int r = e & 31, c = e >> 5;
@@ -489,8 +504,10 @@ __global__ void __launch_bounds__(PB_NT) k_potrs_batched_f64(int n, const double
         __syncthreads();
         if (warp == 0) {
             double xi = lane < w ? x[b0 + lane] : 0.0;
-            for (int j = w - 1; j >= 0; --j) {
-                if (lane == j) xi = xi / blk[j][j];
+            const double ri = lane < w ? 1.0 / blk[lane][lane] : 0.0;
+#pragma unroll 8
+            for (int j = 31; j >= 0; --j) {  // rows at or past w are zero
+                if (lane == j) xi *= ri;
                 const double xj = __shfl_sync(0xffffffffu, xi, j);
                 if (lane < j) xi = fma(-blk[j][lane], xj, xi);
             }
