@@ -62,7 +62,7 @@ __device__ __forceinline__ T wshfl(T v, int src)
 // d += a b, fragments as in panel.cu
 __device__ __forceinline__ void vb_mma(double (&d)[4], double a_up, double a_lo, double b)
 {
-    asm volatile("mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};"
+    asm("mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};"
                  : "+d"(d[0]), "+d"(d[1]), "+d"(d[2]), "+d"(d[3])
                  : "d"(a_up), "d"(a_lo), "d"(b));
 }
