@@ -132,6 +132,11 @@ unsigned long long ddlak_potrs_workspace(int n, int nrhs);
 int ddlak_potrs(char type, char uplo, char side, int n, int nrhs, const void* A, long long lda, void* B,
                 long long ldb, void* work, unsigned long long work_bytes, void* stream);
 
+/* ddlak_potrs enqueued behind a factorization whose device info is *dinfo: does nothing
+ * (B untouched) when that is not 0, so the two need no read-back between them. */
+int ddlak_potrs_after(char type, char uplo, char side, int n, int nrhs, const void* A, long long lda, void* B,
+                      long long ldb, void* work, unsigned long long work_bytes, const int* dinfo, void* stream);
+
 /* ddlak_potrs with its scratch in a fixed device array owned by the library
  * instead of caller memory: no allocation of any kind.  Limits (n <= 65536,
  * nrhs <= 256) are reported by ddlak_potrs_fixed_scratch_limits; larger

@@ -87,8 +87,9 @@ __host__ __device__ constexpr size_t potrs_smem_bytes()
 template <class T, bool UP, bool BT, bool FO = false>
 __global__ void __launch_bounds__(NT) k_potrs_fused(const T* __restrict__ A, long long lda, T* B, long long ldb,
                                                     int n, int nrhs, int nchunks, int* flags, int* ticket,
-                                                    int* status)
+                                                    int* status, const int* __restrict__ skip)
 {
+    if (skip != nullptr && *skip != 0) return;
     using TL = T;
     using R = real_t<T>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -370,8 +371,9 @@ __device__ __forceinline__ bool poll_flag(const int* flag, int* status, bool nea
 template <class TL, class TX, bool UP, bool BT, bool ID, bool FO>
 __global__ void __launch_bounds__(NT, 2) k_potrs_dmma(const TL* __restrict__ A, long long lda, TX* B, long long ldb,
                                                       int n, int nrhs, int nchunks, int* flags, int* ticket,
-                                                      int* status)
+                                                      int* status, const int* __restrict__ skip)
 {
+    if (skip != nullptr && *skip != 0) return;  // the factorization before it failed: B stays
     extern __shared__ __align__(16) unsigned char smem_raw[];
     TL* Lb = reinterpret_cast<TL*>(smem_raw);  // two tiles of RB lines of PD_LD
     double* Ib = reinterpret_cast<double*>(smem_raw + 2 * (size_t)RB * PD_LD * sizeof(TL));  // inverse, row-major
@@ -624,7 +626,7 @@ __global__ void __launch_bounds__(NT, 2) k_potrs_dmma(const TL* __restrict__ A, 
 
 template <class T, bool UP, bool BT, class TL = T, bool ID = false, bool FO = false>
 cudaError_t potrs_launch(const TL* A, long long lda, T* B, long long ldb, int n, int nrhs, int* flags, int* ticket,
-                         int* status, cudaStream_t st)
+                         int* status, cudaStream_t st, const int* skip = nullptr)
 {
     const int N = (int)ceil_div(n, RB);
     const int nchunks = (int)ceil_div(nrhs, RC);
@@ -638,12 +640,12 @@ cudaError_t potrs_launch(const TL* A, long long lda, T* B, long long ldb, int n,
         const size_t smem = potrs_smem_bytes<T>();
         if (cudaError_t e = smem_optin(k_potrs_fused<T, UP, BT, FO>, smem); e != cudaSuccess) return e;
         k_potrs_fused<T, UP, BT, FO><<<(unsigned)grid, NT, smem, st>>>(A, lda, B, ldb, n, nrhs, nchunks, flags, ticket,
-                                                                       status);
+                                                                       status, skip);
     } else {
         const size_t smem = potrs_dmma_smem<TL>();
         if (cudaError_t e = smem_optin(k_potrs_dmma<TL, T, UP, BT, ID, FO>, smem); e != cudaSuccess) return e;
         k_potrs_dmma<TL, T, UP, BT, ID, FO><<<(unsigned)grid, NT, smem, st>>>(A, lda, B, ldb, n, nrhs, nchunks, flags,
-                                                                              ticket, status);
+                                                                              ticket, status, skip);
     }
     note_launches(1);
     return cudaGetLastError();
@@ -651,15 +653,15 @@ cudaError_t potrs_launch(const TL* A, long long lda, T* B, long long ldb, int n,
 
 template <class T>
 cudaError_t potrs_typed(char uplo, char side, int n, int nrhs, const void* A, long long lda, void* B, long long ldb,
-                        int* flags, int* ticket, int* status, cudaStream_t st)
+                        int* flags, int* ticket, int* status, cudaStream_t st, const int* skip)
 {
     const T* a = static_cast<const T*>(A);
     T* b = static_cast<T*>(B);
     const bool up = uplo == 'U', bt = side == 'R';
-    if (up && bt) return potrs_launch<T, true, true>(a, lda, b, ldb, n, nrhs, flags, ticket, status, st);
-    if (up) return potrs_launch<T, true, false>(a, lda, b, ldb, n, nrhs, flags, ticket, status, st);
-    if (bt) return potrs_launch<T, false, true>(a, lda, b, ldb, n, nrhs, flags, ticket, status, st);
-    return potrs_launch<T, false, false>(a, lda, b, ldb, n, nrhs, flags, ticket, status, st);
+    if (up && bt) return potrs_launch<T, true, true>(a, lda, b, ldb, n, nrhs, flags, ticket, status, st, skip);
+    if (up) return potrs_launch<T, true, false>(a, lda, b, ldb, n, nrhs, flags, ticket, status, st, skip);
+    if (bt) return potrs_launch<T, false, true>(a, lda, b, ldb, n, nrhs, flags, ticket, status, st, skip);
+    return potrs_launch<T, false, false>(a, lda, b, ldb, n, nrhs, flags, ticket, status, st, skip);
 }
 
 template <class T>
@@ -679,13 +681,14 @@ cudaError_t forward_typed(char uplo, char side, int n, int nrhs, const void* A, 
 }
 
 cudaError_t potrs_dispatch(char type, char uplo, char side, int n, int nrhs, const void* A, long long lda, void* B,
-                           long long ldb, int* flags, int* ticket, int* status, cudaStream_t st)
+                           long long ldb, int* flags, int* ticket, int* status, cudaStream_t st,
+                           const int* skip = nullptr)
 {
     switch (type) {
-    case 's': return potrs_typed<float>(uplo, side, n, nrhs, A, lda, B, ldb, flags, ticket, status, st);
-    case 'd': return potrs_typed<double>(uplo, side, n, nrhs, A, lda, B, ldb, flags, ticket, status, st);
-    case 'c': return potrs_typed<cf32>(uplo, side, n, nrhs, A, lda, B, ldb, flags, ticket, status, st);
-    case 'z': return potrs_typed<cf64>(uplo, side, n, nrhs, A, lda, B, ldb, flags, ticket, status, st);
+    case 's': return potrs_typed<float>(uplo, side, n, nrhs, A, lda, B, ldb, flags, ticket, status, st, skip);
+    case 'd': return potrs_typed<double>(uplo, side, n, nrhs, A, lda, B, ldb, flags, ticket, status, st, skip);
+    case 'c': return potrs_typed<cf32>(uplo, side, n, nrhs, A, lda, B, ldb, flags, ticket, status, st, skip);
+    case 'z': return potrs_typed<cf64>(uplo, side, n, nrhs, A, lda, B, ldb, flags, ticket, status, st, skip);
     default: return cudaErrorInvalidValue;
     }
 }
@@ -859,8 +862,9 @@ extern "C" int ddlak_potrs_fixed_scratch(char type, char uplo, char side, int n,
                                st);
 }
 
-extern "C" int ddlak_potrs(char type, char uplo, char side, int n, int nrhs, const void* A, long long lda, void* B,
-                           long long ldb, void* work, unsigned long long work_bytes, void* stream)
+extern "C" int ddlak_potrs_after(char type, char uplo, char side, int n, int nrhs, const void* A, long long lda,
+                                 void* B, long long ldb, void* work, unsigned long long work_bytes, const int* dinfo,
+                                 void* stream)
 {
     using namespace ddlak;
     if (n <= 0 || nrhs <= 0) return 0;
@@ -871,7 +875,13 @@ extern "C" int ddlak_potrs(char type, char uplo, char side, int n, int nrhs, con
     int* status = static_cast<int*>(work);
     int* ticket = status + 1;
     int* flags = reinterpret_cast<int*>(static_cast<char*>(work) + 256);
-    return (int)potrs_dispatch(type, uplo, side, n, nrhs, A, lda, B, ldb, flags, ticket, status, st);
+    return (int)potrs_dispatch(type, uplo, side, n, nrhs, A, lda, B, ldb, flags, ticket, status, st, dinfo);
+}
+
+extern "C" int ddlak_potrs(char type, char uplo, char side, int n, int nrhs, const void* A, long long lda, void* B,
+                           long long ldb, void* work, unsigned long long work_bytes, void* stream)
+{
+    return ddlak_potrs_after(type, uplo, side, n, nrhs, A, lda, B, ldb, work, work_bytes, nullptr, stream);
 }
 
 // X = L^-1 B (side 'L', B n x nrhs) or X = B L^-H (side 'R', B nrhs x n), in place,
