@@ -1,0 +1,211 @@
+"""The FP64 tensor-core forms of the factorization, the solves and the batched kernel at the
+sizes where they can go wrong: edges of the 8-, 16-, 64- and 128-wide tiles, odd leading
+dimensions and bases that are only 8-byte aligned, failed pivots on both sides of every tile
+edge, and the FP32 tile products with and without TMA.
+
+Bounds: a Cholesky factor satisfies |A - L L^T| <= (n + 1) u |L||L^T| entrywise (Higham,
+Accuracy and Stability, theorem 10.3); the products here sum in blocks and by reciprocal pivots
+and inverted tiles, each an operation or two more per step, hence the factor 4."""
+import ctypes
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+EPS = {"s": float(np.finfo(np.float32).eps), "d": float(np.finfo(np.float64).eps)}
+NP = {"s": np.float32, "d": np.float64}
+
+
+def _torch():
+    import torch
+
+    return torch
+
+
+def spd(n, seed):
+    g = np.random.default_rng(seed).standard_normal((n, n))
+    return g @ g.T / max(n, 1) + np.eye(n)
+
+
+def device(host, lda, p, shift=0):
+    """Column-major copy with leading dimension lda, its first word `shift` words into the allocation."""
+    torch = _torch()
+    n, m = host.shape
+    flat = np.full(shift + lda * m, np.nan, dtype=NP[p])
+    flat[shift:].reshape(m, lda)[:, :n] = host.T
+    t = torch.from_numpy(flat).cuda()
+    return t, t.data_ptr() + shift * t.element_size()
+
+
+def host(t, n, m, lda, shift=0):
+    return t.cpu().numpy()[shift:].reshape(m, lda)[:, :n].T
+
+
+def potrf(handle, p, uplo, n, ptr, lda):
+    torch = _torch()
+    from libddla_b200 import ddla
+
+    info = torch.full((1,), -7, dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    ddla.potrf(handle, p, uplo, n, ptr, lda, info.data_ptr())
+    handle.synchronize()
+    return int(info[0])
+
+
+def check_factor(a, out, uplo, p):
+    n = a.shape[0]
+    low = np.tril(out) if uplo == "L" else np.triu(out).T
+    low = low.astype(np.float64)
+    bound = 4 * (n + 1) * EPS[p] * (np.abs(low) @ np.abs(low.T)) + np.abs(a) * EPS[p]
+    i = np.tril_indices(n)
+    diff = np.abs(a - low @ low.T)
+    assert np.all(diff[i] <= bound[i]), np.max(diff[i] / bound[i])
+
+
+@pytest.mark.parametrize("p", ["s", "d"])
+@pytest.mark.parametrize("uplo", ["L", "U"])
+@pytest.mark.parametrize("n", [1, 7, 8, 9, 16, 17, 127, 128, 129, 136, 193, 257, 700])
+def test_factor_tile_edges(handle, p, uplo, n):
+    a = spd(n, n).astype(NP[p]).astype(np.float64)
+    for pad, shift in ((0, 0), (1, 0), (2, 1), (5, 3)):
+        poisoned = a.copy()
+        poisoned[np.triu_indices(n, 1) if uplo == "L" else np.tril_indices(n, -1)] = np.nan
+        t, ptr = device(poisoned, n + pad, p, shift)
+        assert potrf(handle, p, uplo, n, ptr, n + pad) == 0
+        out = host(t, n, n, n + pad, shift)
+        other = np.triu_indices(n, 1) if uplo == "L" else np.tril_indices(n, -1)
+        assert np.all(np.isnan(out[other]))
+        check_factor(a, out, uplo, p)
+
+
+@pytest.mark.parametrize("p", ["s", "d"])
+@pytest.mark.parametrize("uplo", ["L", "U"])
+@pytest.mark.parametrize("bad", [0, 6, 7, 8, 63, 64, 127, 128, 199])
+def test_failed_pivot(handle, p, uplo, bad):
+    """info is the failed pivot's order and the columns before it are final."""
+    n = 200
+    a = spd(n, 3).astype(NP[p]).astype(np.float64)
+    want = np.linalg.cholesky(a)
+    b = a.copy()
+    b[bad, bad] = -1.0
+    t, ptr = device(b, n + 1, p)
+    assert potrf(handle, p, uplo, n, ptr, n + 1) == bad + 1
+    out = host(t, n, n, n + 1).astype(np.float64)
+    low = np.tril(out) if uplo == "L" else np.triu(out).T
+    # the block that fails is final in its own rows; the blocks before it in every row
+    rows = n if bad % 128 == 0 else min(n, (bad // 128 + 1) * 128)
+    got, ref = low[:rows, :bad], want[:rows, :bad]
+    keep = np.tril_indices(rows, 0, bad)
+    ok = ref.copy()
+    # row `bad` differs only through the changed diagonal entry, which no earlier column holds
+    assert np.allclose(got[keep], ok[keep], rtol=0, atol=50 * n * EPS[p])
+
+
+@pytest.mark.parametrize("p", ["s", "d"])
+@pytest.mark.parametrize("uplo", ["L", "U"])
+@pytest.mark.parametrize("side", ["L", "R"])
+@pytest.mark.parametrize("n,nrhs", [(1, 1), (63, 8), (64, 9), (65, 16), (129, 17), (700, 3), (701, 33)])
+def test_solve_edges(handle, p, uplo, side, n, nrhs):
+    from libddla_b200 import ddla
+
+    a = spd(n, 5).astype(NP[p]).astype(np.float64)
+    rng = np.random.default_rng(7)
+    b = rng.standard_normal((n, nrhs) if side == "L" else (nrhs, n)).astype(NP[p])
+    ta, pa = device(a, n + 1, p)
+    assert potrf(handle, p, uplo, n, pa, n + 1) == 0
+    ldb = b.shape[0] + 2
+    tb, pb = device(b, ldb, p)
+    wrap = ddla.DistributedMatrix.wrap
+    dA = wrap(handle, pa, n, n, n + 1, NP[p])
+    dB = wrap(handle, pb, b.shape[0], b.shape[1], ldb, NP[p])
+    ddla.ppotrs(dA, dB, uplo=uplo, side=side)
+    x = host(tb, b.shape[0], b.shape[1], ldb).astype(np.float64)
+    res = a @ x - b if side == "L" else x @ a - b
+    # the factor's backward error and that of the two triangular solves, condition number about 5
+    assert np.max(np.abs(res)) <= 40 * (n + 1) * EPS[p] * np.linalg.norm(a, 2) * np.max(np.abs(x))
+
+
+@pytest.mark.parametrize("p", ["s", "d"])
+@pytest.mark.parametrize("variant", [0, 1])
+@pytest.mark.parametrize("solve", [False, True])
+def test_batched_variants(handle, p, variant, solve):
+    """Both block-column widths over every tile edge, odd and padded leading dimensions, matrices that
+    fail on both sides of the edges among them."""
+    torch = _torch()
+    from libddla_b200.ddla import _c_api as C
+
+    orders = [1, 7, 8, 9, 31, 32, 33, 63, 64, 65, 127, 128, 129, 159, 160, 191, 192, 193, 320, 511, 512]
+    fails = [(64, 0), (65, 64), (129, 63), (129, 128), (200, 71), (320, 256), (512, 511)]
+    cases = [(n, None) for n in orders] + fails
+    mats, store, ptrs, rhs, bptr, ldas = [], [], [], [], [], []
+    for i, (n, bad) in enumerate(cases):
+        a = spd(n, 11 + i).astype(NP[p]).astype(np.float64)
+        if bad is not None:
+            a[bad, bad] = -2.0
+        lda = n + i % 4
+        t, ptr = device(a, lda, p, shift=i % 3)
+        b = np.random.default_rng(i).standard_normal((n, 1))
+        tb, pb = device(b, n, p)
+        mats.append(a), store.append(t), ptrs.append(ptr), rhs.append((b, tb)), bptr.append(pb), ldas.append(lda)
+    count = len(cases)
+    up = lambda v, dt: torch.tensor(np.array(v, dtype=dt), device="cuda")
+    dn, dl = up([n for n, _ in cases], np.int32), up(ldas, np.int32)
+    da, db = up(ptrs, np.int64), up(bptr, np.int64)
+    logdet = torch.zeros(count, dtype=torch.float64, device="cuda")
+    info = torch.full((count,), -5, dtype=torch.int32, device="cuda")
+    sel = torch.full((count,), variant, dtype=torch.uint8, device="cuda")
+    counters = torch.zeros(2, dtype=torch.int32, device="cuda")
+    f = C.lib.ddlak_posv_vbatched
+    f.restype = ctypes.c_int
+    f.argtypes = [ctypes.c_char, ctypes.c_int, ctypes.c_int] + [ctypes.c_void_p] * 9 + [ctypes.c_int, ctypes.c_void_p]
+    torch.cuda.synchronize()
+    rc = f(p.encode(), 512, count, dn.data_ptr(), da.data_ptr(), dl.data_ptr(), db.data_ptr() if solve else None,
+           logdet.data_ptr(), info.data_ptr(), None, sel.data_ptr(), counters.data_ptr(), 7,
+           torch.cuda.current_stream().cuda_stream)
+    assert rc == 0
+    torch.cuda.synchronize()
+    for i, (n, bad) in enumerate(cases):
+        out = host(store[i], n, n, ldas[i], i % 3).astype(np.float64)
+        b, tb = rhs[i]
+        x = host(tb, n, 1, n).astype(np.float64)
+        if bad is not None:
+            assert int(info[i]) == bad + 1 and np.isnan(float(logdet[i]))
+            assert np.array_equal(x, b.astype(NP[p]).astype(np.float64))
+            fixed = mats[i].copy()
+            fixed[bad, bad] = 1e3  # any positive definite completion has the same columns before `bad`
+            low = np.linalg.cholesky(fixed)
+            assert np.allclose(np.tril(out)[:, :bad], low[:, :bad], rtol=0, atol=50 * n * EPS[p])
+            continue
+        assert int(info[i]) == 0
+        check_factor(mats[i], out, "L", p)
+        assert np.array_equal(np.triu(out, 1), np.triu(mats[i], 1))
+        want = np.linalg.slogdet(mats[i])[1]
+        assert abs(float(logdet[i]) - want) <= 8 * n * EPS["d"] * n + 1e-12
+        if solve:
+            res = mats[i] @ x - b.astype(NP[p])
+            assert np.max(np.abs(res)) <= 40 * (n + 1) * EPS[p] * np.linalg.norm(mats[i], 2) * np.max(np.abs(x))
+
+
+@pytest.mark.parametrize("n", [1025, 1101, 1536])
+def test_large_fp32_gradient(handle, n):
+    """The FP32 inversion by doubling and the contraction: leading dimensions with TMA (a multiple of
+    4) and without, a last leaf of one row."""
+    torch = _torch()
+    from libddla_b200.ddla import autograd as ag
+
+    g = torch.Generator(device="cuda").manual_seed(n)
+    x = torch.rand(1, n, 2, generator=g, device="cuda", dtype=torch.float32)
+    y = torch.randn(1, n, generator=g, device="cuda", dtype=torch.float32)
+    th = torch.tensor([0.3, 1.0, 0.5], dtype=torch.float64, device="cuda", requires_grad=True)
+    loss = ag.gp_nll(x, y, th, handle)
+    (got,) = torch.autograd.grad(loss.sum(), th)
+    t = th.detach().clone().requires_grad_()
+    xd, yd = x[0].double(), y[0].double()
+    k = t[1] * torch.exp(-torch.cdist(xd, xd).square() / (2 * t[0] ** 2)) + t[2] * torch.eye(n, device="cuda")
+    low = torch.linalg.cholesky(k)
+    want_loss = 0.5 * (yd @ torch.cholesky_solve(yd[:, None], low)[:, 0]) + low.diagonal().log().sum()
+    (want,) = torch.autograd.grad(want_loss, t)
+    # condition number of K + 0.5 I up to about n; errors of n u relative to the largest component
+    assert abs(float(loss) - float(want_loss)) <= 1e-4 * abs(float(want_loss))
+    assert float((got - want).abs().max()) <= 1e-3 * float(want.abs().max())
