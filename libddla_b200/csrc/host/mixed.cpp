@@ -180,9 +180,7 @@ void mixed_core(const DdlaHandle_t& h, char precision, int n, int nrhs, double* 
         detail::DeviceScratch tmp(h, ddlak_bis_inverse_bytes(n));
         ck(ddlak_bis_inverse(n, W, ldw, Dinv, tmp.data(), st), "diagonal block inverses");
         ck(ddlak_bis_inverse_narrow(n, Dinv, Dinv32, st), "FP32 diagonal block inverses");
-    } else {
-        ck(ddlak_inv_diag_blocks(n, W, ldw, Dinv, st), "diagonal block inverses");
-    }
+    }  // else: the fused solve inverts its diagonal blocks itself
     MixedPreconditioner M;
     M.h = h;
     M.n = n;

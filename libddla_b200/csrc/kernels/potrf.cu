@@ -408,12 +408,13 @@ static cudaError_t potrf_typed(char uplo, int n, int G, void* A, long long lda, 
 // L L^T x = b for a batch of factored equal-order FP64 matrices (lower, order
 // <= 1024, one right-hand side each), one CTA per matrix with x in shared
 // memory; log det = 2 sum log l_ii on the way.  Forward, by 32-row blocks: warp
-// 0 solves the block (lane i owns row i; x_j = x_j / l_jj, then broadcast),
+// 0 solves the block (lane i owns row i; x_j times 1 / l_jj, then broadcast),
 // every thread updates its rows below with the block's 32 columns (coalesced
-// column reads).  Backward, by 32-row blocks from the end: each warp forms the
-// dot products of some of the block's columns with the solved x below
-// (coalesced, warp sums), then warp 0 solves the transposed block from a
-// shared copy.  A matrix with info != 0 keeps b and gets log det = NaN.
+// column reads, a row's 32 in flight together).  Backward, by 32-row blocks from
+// the end: each warp forms four of the block's dot products with the solved x
+// below (coalesced, their loads in flight together, warp sums), then warp 0 solves
+// the transposed block from a shared copy.  A matrix with info != 0 keeps b and
+// gets log det = NaN.  What bounds it: load latency over its 64 block steps.
 // ---------------------------------------------------------------------------
 constexpr int PB_NT = 256, PB_NMAX = 1024;
 

@@ -181,7 +181,9 @@ def test_batched_variants(handle, p, variant, solve):
         check_factor(mats[i], out, "L", p)
         assert np.array_equal(np.triu(out, 1), np.triu(mats[i], 1))
         want = np.linalg.slogdet(mats[i])[1]
-        assert abs(float(logdet[i]) - want) <= 8 * n * EPS["d"] * n + 1e-12
+        # the stored factor is that of A + E, |E| <= 4 (n + 1) u |A|; log det moves by at most
+        # trace |A^-1 E| <= n cond(A) 4 (n + 1) u, cond(A) about 5
+        assert abs(float(logdet[i]) - want) <= 20 * n * (n + 1) * EPS[p] + 1e-12
         if solve:
             res = mats[i] @ x - b.astype(NP[p])
             assert np.max(np.abs(res)) <= 40 * (n + 1) * EPS[p] * np.linalg.norm(mats[i], 2) * np.max(np.abs(x))
