@@ -314,30 +314,40 @@ __global__ void __launch_bounds__(NT) k_potrs_fused(const T* __restrict__ A, lon
 }
 
 // ---------------------------------------------------------------------------
-// The same solve for real types on the FP64 tensor cores (m16n8k4 DMMA, FP64
-// arithmetic for FP32 and FP64 storage).  Eight warps: warp w owns rows
+// The same solve for real types on the FP64 tensor cores (DMMA, FP64 arithmetic for FP32
+// and FP64 storage).  Eight warps.  The off-diagonal tiles: warp w owns rows
 // 16 (w % 4) .. + 15 of the block row and right-hand sides 8 (w / 4) .. + 7 of the
 // chunk, as one accumulator fragment.
-//   * Before it joins the chain, a CTA inverts its 64 x 64 diagonal block (8 x 8
-//     tiles by substitution, then the identity's 16-row strips against the block,
-//     as the panel solve of panel.cu), so a link of the chain is two products
-//     (the last off-diagonal tile, the inverse) and no substitution.
+//   * The diagonal block is solved by substitution over 8 x 8 tiles, as the panel solve of
+//     panel.cu: only the 8 x 8 tiles on the diagonal are inverted (before the CTA joins the
+//     chain).  The transpose is kept (rows are right-hand sides), so that a step's
+//     result is the next product's operand without a shuffle: warp w owns rows
+//     16 (w / 2) .. + 15 for right-hand sides 8 (w % 2) .. + 7 and hands its solution to the
+//     other three warps of its right-hand sides through shared memory.  The inverse
+//     of the whole 64 x 64 block in place of this is not backward stable: for
+//     a squared-exponential kernel on a line, condition 1e14, n = 256, the backward error
+//     was 1e-12 with 64-row inverses, 1e-15 with 16-row ones and 4e-17 with 8-row
+//     ones, as by substitution.
 //   * One thread polls the flag of the block needed; every warp reads that block's
 //     solution straight into its operand fragments; the next one is fetched under
 //     the current product when its flag is already up.
-// What bounds it: the chain of n / 64 links per direction.  Measured (one call, factor
-// and flags in place) against the substitution form: n = 2048, 16 right-hand sides 240
-// against 556 us; n = 5003, 3 of them 0.56 against 1.38 ms; n = 16384, 64 of them 4.8
-// against 6.6 ms.
+// What bounds it: the chain of n / 64 links per direction.  Measured (one call, factor and flags
+// in place) against the substitution form by warps, FP64: n = 2048, 16 right-hand sides 310
+// against 556 us; n = 5003, 16 of them 0.92 against 1.41 ms; n = 8192, 64 of them 1.66
+// against 2.57 ms (with whole inverses 261 us, 0.85 ms and 1.61 ms).
 // ---------------------------------------------------------------------------
 constexpr int PD_LD = RB + 4;  // 4 mod 16 doubles: conflict-free fragment reads either way round
 constexpr int PD_LDX = RC + 4;
 
+constexpr int PD_XT = RB / 8 * 64;  // doubles of one half's published solution: 8 tiles, 2 a lane
+
+// two tiles of the ring (the block row's right-hand sides and the published solution of the
+// diagonal step take their place afterwards), the diagonal block in FP64
 template <class TL>
 __host__ __device__ constexpr size_t potrs_dmma_smem()
 {
-    return 2 * (size_t)RB * PD_LD * sizeof(TL) + (size_t)RB * PD_LD * sizeof(double) +
-           (sizeof(TL) < 8 ? (size_t)RB * PD_LDX * sizeof(double) : 0);
+    static_assert(2 * RB * PD_LD * sizeof(TL) >= (RB * PD_LDX + 2 * PD_XT) * sizeof(double), "diagonal step");
+    return 2 * (size_t)RB * PD_LD * sizeof(TL) + (size_t)RB * PD_LD * sizeof(double);
 }
 
 __device__ __forceinline__ void pd_mma(double (&d)[4], double a_up, double a_lo, double b)
@@ -345,6 +355,16 @@ __device__ __forceinline__ void pd_mma(double (&d)[4], double a_up, double a_lo,
     asm("mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};"
                  : "+d"(d[0]), "+d"(d[1]), "+d"(d[2]), "+d"(d[3])
                  : "d"(a_up), "d"(a_lo), "d"(b));
+}
+
+// d += a b with m8n8k4: lane (g = lane / 4, q = lane % 4) supplies A(g, q) and B(q, g) and holds
+// D(g, 2q), D(g, 2q + 1); these two are the A operands of a next product over k in the
+// order {0, 2, 4, 6}, {1, 3, 5, 7}.
+__device__ __forceinline__ void pd_mma8(double (&d)[2], double a, double b)
+{
+    asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+        : "+d"(d[0]), "+d"(d[1])
+        : "d"(a), "d"(b));
 }
 
 // One thread: until *flag >= 1 or the budget runs out (DDLAK_WAIT_TIMEOUT in *status, false).
@@ -376,9 +396,9 @@ __global__ void __launch_bounds__(NT, 2) k_potrs_dmma(const TL* __restrict__ A, 
     if (skip != nullptr && *skip != 0) return;  // the factorization before it failed: B stays
     extern __shared__ __align__(16) unsigned char smem_raw[];
     TL* Lb = reinterpret_cast<TL*>(smem_raw);  // two tiles of RB lines of PD_LD
-    double* Ib = reinterpret_cast<double*>(smem_raw + 2 * (size_t)RB * PD_LD * sizeof(TL));  // inverse, row-major
-    // the block row's right-hand sides between the two products: over the (then free) tiles
-    double* Xs = sizeof(TL) < 8 ? Ib + RB * PD_LD : reinterpret_cast<double*>(smem_raw);
+    double* Db = reinterpret_cast<double*>(smem_raw + 2 * (size_t)RB * PD_LD * sizeof(TL));  // the diagonal block
+    double* Xs = reinterpret_cast<double*>(smem_raw);  // the block row's right-hand sides, over the (then free) tiles
+    double* Xt = Xs + RB * PD_LDX;                     // and the diagonal step's solution, a tile's fragment at a time
     __shared__ __align__(16) double T8[8 * 64];  // inverses of the diagonal 8 x 8 tiles
     __shared__ int s_t, s_next;
     if (threadIdx.x == 0) s_t = atomicAdd(ticket, 1);
@@ -426,67 +446,43 @@ __global__ void __launch_bounds__(NT, 2) k_potrs_dmma(const TL* __restrict__ A, 
             }
         }
     };
-    // the diagonal block into tile 0: lines [c][r] ('L') or [r][c] ('U'); its strict upper part is not used
+    // the diagonal block: lines [c][r] ('L') or [r][c] ('U'), zero in its strict upper part and
+    // past the matrix; FP32 storage by way of tile 0
     {
         const TL* src0 = A + i0 + i0 * lda;
+        TL* dst = sizeof(TL) == 8 ? reinterpret_cast<TL*>(Db) : Lb;
         for (int idx = threadIdx.x; idx < RB * RB; idx += NT) {
             const int l = idx >> 6, w = idx & (RB - 1);
             const bool in = l < nrows && w < nrows && (UP ? w <= l : w >= l);
-            cp_async_elem<sizeof(TL)>(Lb + l * PD_LD + w, in ? src0 + l * lda + w : A, in);
+            cp_async_elem<sizeof(TL)>(dst + l * PD_LD + w, in ? src0 + l * lda + w : A, in);
         }
     }
     cp_commit();
     if (nvisit > 0) issue_tile(visit(0), 1);
     cp_commit();
-
-    // ---- inverse of the diagonal block (padded with the identity) --------------------
-    auto lval = [&](int r, int c) { return (double)(UP ? Lb[r * PD_LD + c] : Lb[c * PD_LD + r]); };
     cp_wait<1>();
-    for (int idx = threadIdx.x; idx < RB * PD_LD; idx += NT) Ib[idx] = 0.0;
     __syncthreads();
+    if constexpr (sizeof(TL) < 8) {
+        for (int idx = threadIdx.x; idx < RB * RB; idx += NT) {
+            const int l = idx >> 6, w = idx & (RB - 1);
+            Db[l * PD_LD + w] = (double)Lb[l * PD_LD + w];
+        }
+        __syncthreads();
+    }
     if (threadIdx.x < 64) {
-        // column c of diagonal tile b's inverse
+        // column c of diagonal tile b's inverse (rows past the matrix: the identity)
         const int b = threadIdx.x >> 3, c = threadIdx.x & 7;
+        const double* tile = Db + 8 * b * (PD_LD + 1);
         double y[8];
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
             double v = i == c ? 1.0 : 0.0;
 #pragma unroll
-            for (int k = 0; k < i; ++k) v = fma(-lval(8 * b + i, 8 * b + k), y[k], v);
-            y[i] = 8 * b + i < nrows ? v / lval(8 * b + i, 8 * b + i) : v;
+            for (int k = 0; k < i; ++k) v = fma(-tile[UP ? i * PD_LD + k : k * PD_LD + i], y[k], v);
+            y[i] = 8 * b + i < nrows ? v / tile[i * (PD_LD + 1)] : v;
         }
 #pragma unroll
         for (int i = 0; i < 8; ++i) T8[b * 64 + i * 8 + c] = y[i];
-    }
-    __syncthreads();
-    if (warp < 4) {
-        // X L^T = I by 16-row strips (panel.cu): X(i, m) = (L^-1)(m, i)
-        double C[8][4];
-#pragma unroll
-        for (int l = 0; l < 8; ++l)
-#pragma unroll
-            for (int h = 0; h < 2; ++h)
-#pragma unroll
-                for (int e = 0; e < 2; ++e) C[l][2 * h + e] = row + 8 * h == 8 * l + 2 * q + e ? 1.0 : 0.0;
-#pragma unroll 1
-        for (int j = 0; j < 8; ++j) {
-            double X[4] = {0.0, 0.0, 0.0, 0.0};
-            pd_mma(X, C[0][0], C[0][2], T8[j * 64 + g * 8 + 2 * q]);
-            pd_mma(X, C[0][1], C[0][3], T8[j * 64 + g * 8 + 2 * q + 1]);
-#pragma unroll
-            for (int h = 0; h < 2; ++h)
-#pragma unroll
-                for (int e = 0; e < 2; ++e) Ib[(8 * j + 2 * q + e) * PD_LD + row + 8 * h] = X[2 * h + e];
-#pragma unroll
-            for (int l = 1; l < 8; ++l) {
-                if (l > 7 - j) break;
-                double D[4] = {C[l][0], C[l][1], C[l][2], C[l][3]};
-                pd_mma(D, -X[0], -X[2], lval(8 * (j + l) + g, 8 * j + 2 * q));
-                pd_mma(D, -X[1], -X[3], lval(8 * (j + l) + g, 8 * j + 2 * q + 1));
-#pragma unroll
-                for (int e = 0; e < 4; ++e) C[l - 1][e] = D[e];
-            }
-        }
     }
     __syncthreads();
 
@@ -581,6 +577,23 @@ __global__ void __launch_bounds__(NT, 2) k_potrs_dmma(const TL* __restrict__ A, 
         __syncthreads();  // the tile is free
     }
     cp_wait<0>();
+
+    // ---- the diagonal block: rows 16 w .. of right-hand sides 8 h .., transposed ------
+    // forward x L^T = c through the tiles 0 .. 7, backward x L = c through 7 .. 0
+    const int h = warp & 1, w = warp >> 1;
+    const bool mine = r0 + 8 * h < nrhs;  // uniform over the four warps of a half
+    const int ta = 2 * w + (fwd ? 0 : 1), tb = 2 * w + (fwd ? 1 : 0);  // this warp's first and second tile
+    // operand of C_l -= X_j (.): L_lj^T (forward) or L_jl (backward), entries (2q + e, g)
+    auto off = [&](int l, int j) {
+        const double* p = Db + (p1 ? (8 * j + 2 * q) * PD_LD + 8 * l + g : (8 * l + g) * PD_LD + 8 * j + 2 * q);
+        return make_double2(p[0], p[p1 ? PD_LD : 1]);
+    };
+    const int inv_c = fwd ? 8 : 1, inv_m = fwd ? 1 : 8;
+    auto inv = [&](int j) {
+        const double* p = T8 + j * 64 + g * inv_c + 2 * q * inv_m;
+        return make_double2(p[0], p[inv_m]);
+    };
+    const double2 va = inv(ta), vb = inv(tb), vab = off(tb, ta);
     {
         double* p = Xs + row * PD_LDX + 8 * (warp >> 2) + 2 * q;
         p[0] = acc[0] + acc2[0];
@@ -589,36 +602,61 @@ __global__ void __launch_bounds__(NT, 2) k_potrs_dmma(const TL* __restrict__ A, 
         p[8 * PD_LDX + 1] = acc[3] + acc2[3];
     }
     __syncthreads();
-    if (live) {
-        // x = Inv acc (forward) or Inv^T acc (backward); Inv is zero above its diagonal
-        double x[4] = {0.0, 0.0, 0.0, 0.0}, x2[4] = {0.0, 0.0, 0.0, 0.0};
-        const double* xb = Xs + 8 * (warp >> 2) + g;
-        const int s = warp & 3;
-        if (fwd) {
+    if (mine) {
+        const double* xa = Xs + (8 * ta + 2 * q) * PD_LDX + 8 * h + g;
+        const double* xb = Xs + (8 * tb + 2 * q) * PD_LDX + 8 * h + g;
+        double Ca[2] = {xa[0], xa[PD_LDX]}, Cb[2] = {xb[0], xb[PD_LDX]};
+        double Xa[2] = {0.0, 0.0}, Xb[2] = {0.0, 0.0};
+        double* xt = Xt + h * PD_XT + 2 * lane;
+        auto solve = [&](const double (&C)[2], double2 v, double (&X)[2]) {
+            X[0] = X[1] = 0.0;
+            pd_mma8(X, C[0], v.x);
+            pd_mma8(X, C[1], v.y);
+        };
+        auto update = [&](double (&C)[2], double x0, double x1, double2 v) {
+            pd_mma8(C, -x0, v.x);
+            pd_mma8(C, -x1, v.y);
+        };
 #pragma unroll
-            for (int m = 0; m < RB / 4; m += 2) {
-                if (m >= 4 * (s + 1)) break;
-                const double* p = Ib + row * PD_LD + 4 * m + q;
-                pd_mma(x, p[0], p[8 * PD_LD], xb[(4 * m + q) * PD_LDX]);
-                pd_mma(x2, p[4], p[8 * PD_LD + 4], xb[(4 * m + 4 + q) * PD_LDX]);
+        for (int s = 0; s < RB / 16; ++s) {
+            const int jb = fwd ? s : RB / 16 - 1 - s;  // the block solved in this step
+            const int ja = 2 * jb + (fwd ? 0 : 1), jc = 2 * jb + (fwd ? 1 : 0);
+            double2 o[4];
+            if (w == jb) {
+                solve(Ca, va, Xa);
+                update(Cb, Xa[0], Xa[1], vab);
+                solve(Cb, vb, Xb);
+                if (s + 1 < RB / 16) {
+                    *reinterpret_cast<double2*>(xt + ta * 64) = make_double2(Xa[0], Xa[1]);
+                    *reinterpret_cast<double2*>(xt + tb * 64) = make_double2(Xb[0], Xb[1]);
+                }
             }
-        } else {
-#pragma unroll
-            for (int m = 0; m < RB / 4; m += 2) {
-                if (m < 4 * s) continue;
-                const double* p = Ib + (4 * m + q) * PD_LD + row;
-                pd_mma(x, p[0], p[8], xb[(4 * m + q) * PD_LDX]);
-                pd_mma(x2, p[4 * PD_LD], p[4 * PD_LD + 8], xb[(4 * m + 4 + q) * PD_LDX]);
+            if (s + 1 == RB / 16) break;
+            const bool below = fwd ? w > jb : w < jb;
+            if (below) {  // the operands while the block is being solved
+                o[0] = off(ta, ja);
+                o[1] = off(ta, jc);
+                o[2] = off(tb, ja);
+                o[3] = off(tb, jc);
+            }
+            if (h == 0) asm volatile("bar.sync 1, 128;" ::: "memory");
+            else asm volatile("bar.sync 2, 128;" ::: "memory");
+            if (below) {
+                const double2 x0 = *reinterpret_cast<const double2*>(xt + ja * 64);
+                const double2 x1 = *reinterpret_cast<const double2*>(xt + jc * 64);
+                update(Ca, x0.x, x0.y, o[0]);
+                update(Cb, x0.x, x0.y, o[2]);
+                update(Ca, x1.x, x1.y, o[1]);
+                update(Cb, x1.x, x1.y, o[3]);
             }
         }
+        const long long r = r0 + 8 * h + g;
 #pragma unroll
-        for (int h = 0; h < 2; ++h)
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                const long long r = rc + 2 * q + e;
-                if (row + 8 * h < nrows && r < nrhs)
-                    x_st<TX, BT>(B, ldb, i0 + row + 8 * h, r, (TX)(x[2 * h + e] + x2[2 * h + e]));
-            }
+        for (int e = 0; e < 2; ++e) {
+            const int ia = 8 * ta + 2 * q + e, ib = 8 * tb + 2 * q + e;
+            if (r < nrhs && ia < nrows) x_st<TX, BT>(B, ldb, i0 + ia, r, (TX)Xa[e]);
+            if (r < nrhs && ib < nrows) x_st<TX, BT>(B, ldb, i0 + ib, r, (TX)Xb[e]);
+        }
     }
     __syncthreads();
     if (threadIdx.x == 0) st_release(&cflags[fwd ? blk : N + blk], 1);  // orders the CTA's stores too
