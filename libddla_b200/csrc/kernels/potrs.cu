@@ -328,26 +328,34 @@ __global__ void __launch_bounds__(NT) k_potrs_fused(const T* __restrict__ A, lon
 //     a squared-exponential kernel on a line, condition 1e14, n = 256, the backward error
 //     was 1e-12 with 64-row inverses, 1e-15 with 16-row ones and 4e-17 with 8-row
 //     ones, as by substitution.
-//   * One thread polls the flag of the block needed; every warp reads that block's
-//     solution straight into its operand fragments; the next one is fetched under
-//     the current product when its flag is already up.
-// What bounds it: the chain of n / 64 links per direction.  Measured (one call, factor and flags
-// in place) against the substitution form by warps, FP64: n = 2048, 16 right-hand sides 310
-// against 556 us; n = 5003, 16 of them 0.92 against 1.41 ms; n = 8192, 64 of them 1.66
-// against 2.57 ms (with whole inverses 261 us, 0.85 ms and 1.61 ms).
+//   * One thread polls the flag of the block needed; behind it a warp looks how many of the
+//     next 32 blocks are up too, so that blocks known to be up cost no look and no fence.
+//     A block's solution goes through shared memory, four entries a thread, fetched under
+//     the product before it when its flag is up.  (With a look per block, and the solution
+//     read by each of the four warps that need it in 16 loads a thread, n = 5003 with as many
+//     right-hand sides took 47.7 ms, 18.4 now.)
+// What bounds it: with few right-hand sides the chain of n / 64 links per direction; with many
+// the latency of a visit (tile, solution, product, two barriers), two CTAs per SM over it.
+// Measured (one call, factor and flags in place) against the substitution form by warps, FP64:
+// n = 2048, 16 right-hand sides 256 against 556 us, 2048 of them 1.26 against 2.42 ms;
+// n = 5003, 16 of them 0.65 against 1.41 ms, 5003 of them 18.4 against 32.8 ms; n = 8192,
+// 64 of them 1.10 against 2.57 ms.  FP32: n = 5003, 16 of them 0.61 against 1.11 ms, 5003 of
+// them 16.5 against 24.2 ms.
 // ---------------------------------------------------------------------------
 constexpr int PD_LD = RB + 4;  // 4 mod 16 doubles: conflict-free fragment reads either way round
 constexpr int PD_LDX = RC + 4;
+constexpr int PD_LDV = RB + 4;
 
 constexpr int PD_XT = RB / 8 * 64;  // doubles of one half's published solution: 8 tiles, 2 a lane
 
 // two tiles of the ring (the block row's right-hand sides and the published solution of the
-// diagonal step take their place afterwards), the diagonal block in FP64
+// diagonal step take their place afterwards), the diagonal block in FP64, another block
+// row's solution
 template <class TL>
 __host__ __device__ constexpr size_t potrs_dmma_smem()
 {
     static_assert(2 * RB * PD_LD * sizeof(TL) >= (RB * PD_LDX + 2 * PD_XT) * sizeof(double), "diagonal step");
-    return 2 * (size_t)RB * PD_LD * sizeof(TL) + (size_t)RB * PD_LD * sizeof(double);
+    return 2 * (size_t)RB * PD_LD * sizeof(TL) + (size_t)(RB * PD_LD + RC * PD_LDV) * sizeof(double);
 }
 
 __device__ __forceinline__ void pd_mma(double (&d)[4], double a_up, double a_lo, double b)
@@ -399,8 +407,8 @@ __global__ void __launch_bounds__(NT, 2) k_potrs_dmma(const TL* __restrict__ A, 
     double* Db = reinterpret_cast<double*>(smem_raw + 2 * (size_t)RB * PD_LD * sizeof(TL));  // the diagonal block
     double* Xs = reinterpret_cast<double*>(smem_raw);  // the block row's right-hand sides, over the (then free) tiles
     double* Xt = Xs + RB * PD_LDX;                     // and the diagonal step's solution, a tile's fragment at a time
-    __shared__ __align__(16) double T8[8 * 64];  // inverses of the diagonal 8 x 8 tiles
-    __shared__ int s_t, s_next;
+    double* Xv = Db + RB * PD_LD;                      // the other block row's solution, negated: [r][k]
+    __shared__ int s_t, s_ready;
     if (threadIdx.x == 0) s_t = atomicAdd(ticket, 1);
     __syncthreads();
     const int N = (int)ceil_div(n, RB);
@@ -470,9 +478,9 @@ __global__ void __launch_bounds__(NT, 2) k_potrs_dmma(const TL* __restrict__ A, 
         __syncthreads();
     }
     if (threadIdx.x < 64) {
-        // column c of diagonal tile b's inverse (rows past the matrix: the identity)
+        // column c of diagonal tile b's inverse, in the tile's place (rows past the matrix: the identity)
         const int b = threadIdx.x >> 3, c = threadIdx.x & 7;
-        const double* tile = Db + 8 * b * (PD_LD + 1);
+        double* tile = Db + 8 * b * (PD_LD + 1);
         double y[8];
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
@@ -481,8 +489,9 @@ __global__ void __launch_bounds__(NT, 2) k_potrs_dmma(const TL* __restrict__ A, 
             for (int k = 0; k < i; ++k) v = fma(-tile[UP ? i * PD_LD + k : k * PD_LD + i], y[k], v);
             y[i] = 8 * b + i < nrows ? v / tile[i * (PD_LD + 1)] : v;
         }
+        __syncwarp();  // a tile's eight threads are in one warp
 #pragma unroll
-        for (int i = 0; i < 8; ++i) T8[b * 64 + i * 8 + c] = y[i];
+        for (int i = 0; i < 8; ++i) tile[UP ? i * PD_LD + c : c * PD_LD + i] = y[i];
     }
     __syncthreads();
 
@@ -514,67 +523,74 @@ __global__ void __launch_bounds__(NT, 2) k_potrs_dmma(const TL* __restrict__ A, 
                 acc[2 * h + e] = in ? v : 0.0;
             }
         }
-    double xr[RB / 4];  // operand fragments of the other block's solution: X(k = 4 m + q, r = g), negated
-    bool pre = false;
+    // The other block's solution: four entries a thread (of B(0, 0) where there is nothing to
+    // load: unconditional, so that the loads are in flight together), by way of shared memory
+    double xv[4];
+    auto xk = [](int i) { return BT ? (threadIdx.x + NT * i) / RC : (threadIdx.x + NT * i) % RB; };
+    auto xr = [](int i) { return BT ? (threadIdx.x + NT * i) % RC : (threadIdx.x + NT * i) / RB; };
     auto load_x = [&](int j) {
         const long long j0 = (long long)j * RB;
 #pragma unroll
-        for (int m = 0; m < RB / 4; ++m) {
-            // unconditional (of B(0, 0) where there is nothing to load): as branches the 16 loads
-            // took their latencies one after the other, 5000 of a link's 11000 clocks
-            const long long k = j0 + 4 * m + q;
-            const bool in = k < n && rc + g < nrhs;
-            const double v = (double)x_ld_cg<TX, BT>(B, ldb, in ? k : 0, in ? rc + g : 0);
-            xr[m] = in ? -v : 0.0;
+        for (int i = 0; i < RB * RC / NT; ++i) {
+            const long long k = j0 + xk(i), r = r0 + xr(i);
+            const bool in = k < n && r < nrhs;
+            const double v = (double)x_ld_cg<TX, BT>(B, ldb, in ? k : 0, in ? r : 0);
+            xv[i] = in ? -v : 0.0;
         }
     };
+    int ready = 0;  // visits whose solution is known to be published
     for (int v = 0; v < nvisit; ++v) {
         if (v + 1 < nvisit) issue_tile(visit(v + 1), v & 1);  // tile v sits in buffer (v + 1) & 1
         cp_commit();
-        if (!pre) {
+        if (v >= ready) {
             const int j = visit(v);
             wait_flag(&cflags[fwd ? j : N + j], v + 1 == nvisit);
             if (fail) {
                 cp_wait<0>();
                 return;
             }
-            if (live) load_x(j);
+            load_x(j);
+            ready = v + 1;
         }
-        if (threadIdx.x == 0) {
+#pragma unroll
+        for (int i = 0; i < RB * RC / NT; ++i) Xv[xr(i) * PD_LDV + xk(i)] = xv[i];
+        const bool look = v + 1 < nvisit && ready == v + 1;  // uniform over the CTA
+        if (look && warp == 0) {
+            // how many of the next 32 visits' solutions are up
+            const int vn = v + 1 + lane;
             bool up = false;
-            if (v + 1 < nvisit) {
-                const int j = visit(v + 1);
+            if (vn < nvisit) {
+                const int j = visit(vn);
                 up = ld_relaxed(&cflags[fwd ? j : N + j]) >= 1;
-                if (up) __threadfence();
             }
-            s_next = up;
+            const unsigned m = __ballot_sync(0xffffffffu, up);
+            if (m & 1) __threadfence();
+            if (lane == 0) s_ready = v + 1 + (m == 0xffffffffu ? 32 : __ffs(~m) - 1);
         }
         cp_wait<1>();
         __syncthreads();
-        pre = s_next != 0;
+        if (look) ready = s_ready;
+        if (v + 1 < ready) load_x(visit(v + 1));  // under the product
         if (live) {
-            double b[RB / 4];
-#pragma unroll
-            for (int m = 0; m < RB / 4; ++m) b[m] = xr[m];
-            if (pre) load_x(visit(v + 1));
             const TL* Lt = Lb + ((v + 1) & 1) * RB * PD_LD;
+            const double* b = Xv + (8 * (warp >> 2) + g) * PD_LDV + q;
             if (p1) {
 #pragma unroll
                 for (int m = 0; m < RB / 4; m += 2) {
                     const TL* p = Lt + (4 * m + q) * PD_LD + row;
-                    pd_mma(acc, (double)p[0], (double)p[8], b[m]);
-                    pd_mma(acc2, (double)p[4 * PD_LD], (double)p[4 * PD_LD + 8], b[m + 1]);
+                    pd_mma(acc, (double)p[0], (double)p[8], b[4 * m]);
+                    pd_mma(acc2, (double)p[4 * PD_LD], (double)p[4 * PD_LD + 8], b[4 * m + 4]);
                 }
             } else {
 #pragma unroll
                 for (int m = 0; m < RB / 4; m += 2) {
                     const TL* p = Lt + row * PD_LD + 4 * m + q;
-                    pd_mma(acc, (double)p[0], (double)p[8 * PD_LD], b[m]);
-                    pd_mma(acc2, (double)p[4], (double)p[8 * PD_LD + 4], b[m + 1]);
+                    pd_mma(acc, (double)p[0], (double)p[8 * PD_LD], b[4 * m]);
+                    pd_mma(acc2, (double)p[4], (double)p[8 * PD_LD + 4], b[4 * m + 4]);
                 }
             }
         }
-        __syncthreads();  // the tile is free
+        __syncthreads();  // the tile and Xv are free
     }
     cp_wait<0>();
 
@@ -588,12 +604,7 @@ __global__ void __launch_bounds__(NT, 2) k_potrs_dmma(const TL* __restrict__ A, 
         const double* p = Db + (p1 ? (8 * j + 2 * q) * PD_LD + 8 * l + g : (8 * l + g) * PD_LD + 8 * j + 2 * q);
         return make_double2(p[0], p[p1 ? PD_LD : 1]);
     };
-    const int inv_c = fwd ? 8 : 1, inv_m = fwd ? 1 : 8;
-    auto inv = [&](int j) {
-        const double* p = T8 + j * 64 + g * inv_c + 2 * q * inv_m;
-        return make_double2(p[0], p[inv_m]);
-    };
-    const double2 va = inv(ta), vb = inv(tb), vab = off(tb, ta);
+    const double2 va = off(ta, ta), vb = off(tb, tb), vab = off(tb, ta);  // (inverses on the diagonal)
     {
         double* p = Xs + row * PD_LDX + 8 * (warp >> 2) + 2 * q;
         p[0] = acc[0] + acc2[0];

@@ -126,6 +126,27 @@ def test_solve_edges(handle, p, uplo, side, n, nrhs):
     assert np.max(np.abs(res)) <= 40 * (n + 1) * EPS[p] * np.linalg.norm(a, 2) * np.max(np.abs(x))
 
 
+@pytest.mark.parametrize("p", ["s", "d"])
+@pytest.mark.parametrize("uplo,side", [("L", "L"), ("U", "R")])
+@pytest.mark.parametrize("n,nrhs", [(2240, 33), (2497, 40)])
+def test_solve_many_blocks(handle, p, uplo, side, n, nrhs):
+    """Block rows with more than 32 others before them, a last chunk of one right-hand side."""
+    from libddla_b200 import ddla
+
+    a = spd(n, 21).astype(NP[p]).astype(np.float64)
+    b = np.random.default_rng(8).standard_normal((n, nrhs) if side == "L" else (nrhs, n)).astype(NP[p])
+    ta, pa = device(a, n, p)
+    assert potrf(handle, p, uplo, n, pa, n) == 0
+    tb, pb = device(b, b.shape[0] + 1, p)
+    wrap = ddla.DistributedMatrix.wrap
+    dA = wrap(handle, pa, n, n, n, NP[p])
+    ddla.ppotrs(dA, wrap(handle, pb, b.shape[0], b.shape[1], b.shape[0] + 1, NP[p]), uplo=uplo, side=side)
+    x = host(tb, b.shape[0], b.shape[1], b.shape[0] + 1).astype(np.float64)
+    res = a @ x - b if side == "L" else x @ a - b
+    # as test_solve_edges
+    assert np.max(np.abs(res)) <= 40 * (n + 1) * EPS[p] * np.linalg.norm(a, 2) * np.max(np.abs(x))
+
+
 @pytest.mark.parametrize("uplo", ["L", "U"])
 @pytest.mark.parametrize("side", ["L", "R"])
 @pytest.mark.parametrize("n,noise", [(64, 1e-12), (256, 1e-8), (256, 1e-12), (700, 1e-10)])
