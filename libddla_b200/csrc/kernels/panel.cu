@@ -40,6 +40,22 @@ __device__ __forceinline__ void dmma4(double (&d)[4], const double (&c)[4], doub
                  : "d"(a_up), "d"(a_lo), "d"(b), "d"(c[0]), "d"(c[1]), "d"(c[2]), "d"(c[3]));
 }
 
+// X = C Inv^T for one tile of a strip (Inv row-major)
+__device__ __forceinline__ void tile_solve(double (&X)[4], const double (&C)[4], const double* Inv, int g, int q)
+{
+    const double2 b = *reinterpret_cast<const double2*>(&Inv[g * 8 + 2 * q]);
+    const double z[4] = {0.0, 0.0, 0.0, 0.0};
+    double Y[4];
+    dmma4(Y, z, C[0], C[2], b.x);
+    dmma4(X, Y, C[1], C[3], b.y);
+}
+// the same where C holds NaN or infinities
+__device__ __forceinline__ void tile_solve_rows(double (&X)[4], const double (&C)[4], const double* Inv, int lane)
+{
+    const double2 u = tri_row(C[0], C[1], Inv, 1, 8, true, lane), v = tri_row(C[2], C[3], Inv, 1, 8, true, lane);
+    X[0] = u.x, X[1] = u.y, X[2] = v.x, X[3] = v.y;
+}
+
 // C_(l-1) = C_l - X B_l^T for the strip's tiles L0 <= l < L0 + G, as straight-line code: all the
 // operand loads, then the first products, then the second ones, so that neither the loads'
 // nor the products' latency is exposed (with a branch per tile a product took 59 clocks).
@@ -159,6 +175,7 @@ __global__ void __launch_bounds__(DG_THREADS, 1) k_potrf_diag_dmma(S* __restrict
                 if (r >= 8 * (j + 1) && r < nbk && c < good) Ab[lpos<UP>(lda, r, 8 * j + c)] = (S)X[2 * h + e];
             }
     };
+    const bool odd = any_nonfinite(C);
     double X[4] = {0.0, 0.0, 0.0, 0.0};
     int fail = 0;
 #pragma unroll 1
@@ -173,11 +190,9 @@ __global__ void __launch_bounds__(DG_THREADS, 1) k_potrf_diag_dmma(S* __restrict
         bar_sync<2, DG_THREADS>();      // Inv and s_fail are in
         fail = s_fail;
         if (cnt >= 0) {
-            const double2 b = *reinterpret_cast<const double2*>(&Inv[g * 8 + 2 * q]);
-            const double z[4] = {0.0, 0.0, 0.0, 0.0};
-            double Y[4];
-            dmma4(Y, z, C[0][0], C[0][2], b.x);
-            dmma4(X, Y, C[0][1], C[0][3], b.y);
+            tile_solve(X, C[0], Inv, g, q);
+            // (a failed pivot may have put NaN in its column of every row)
+            if (odd || fail) tile_solve_rows(X, C[0], Inv, lane);
             *reinterpret_cast<double2*>(&Xs[r_up * 8 + 2 * q]) = make_double2(X[0], X[1]);
             *reinterpret_cast<double2*>(&Xs[r_lo * 8 + 2 * q]) = make_double2(X[2], X[3]);
         }
@@ -333,33 +348,33 @@ __global__ void __launch_bounds__(TR_NT) k_trsm_panel_dmma(S* __restrict__ A, lo
     const int unit = ((q ^ (g >> 1)) << 1) + g * 8;
     S* out = A + lpos<UP>(lda, r_up, k0 + 2 * q);  // this lane's entries of the step's columns
     const long long e_col = UP ? 1 : lda, e_row = UP ? 8 * lda : 8, e_step = UP ? 8 : 8 * lda;
+    auto run = [&](auto odd) {
 #pragma unroll 1
-    for (int j = 0; j < steps; ++j) {
-        double X[4];
-        {
-            const double2 b = *reinterpret_cast<const double2*>(&Inv[j * 64 + g * 8 + 2 * q]);
-            const double z[4] = {0.0, 0.0, 0.0, 0.0};
-            double Y[4];
-            dmma4(Y, z, C[0][0], C[0][2], b.x);
-            dmma4(X, Y, C[0][1], C[0][3], b.y);
-        }
-        const int cnt = steps - 1 - j;
-        auto tile = [&](int l) {
-            const int r = j + l < PN_TILES ? j + l : PN_TILES - 1;
-            return *reinterpret_cast<const double2*>(&Lt[tr_tile(r, j) + unit]);
-        };
+        for (int j = 0; j < steps; ++j) {
+            double X[4];
+            if constexpr (decltype(odd)::value) tile_solve_rows(X, C[0], Inv + j * 64, lane);
+            else tile_solve(X, C[0], Inv + j * 64, g, q);
+            const int cnt = steps - 1 - j;
+            auto tile = [&](int l) {
+                const int r = j + l < PN_TILES ? j + l : PN_TILES - 1;
+                return *reinterpret_cast<const double2*>(&Lt[tr_tile(r, j) + unit]);
+            };
 #pragma unroll
-        for (int e = 0; e < 2; ++e) {
-            if (8 * j + 2 * q + e < nbk) {
-                if (r_up < n) out[e * e_col] = (S)X[e];
-                if (r_lo < n) out[e * e_col + e_row] = (S)X[2 + e];
+            for (int e = 0; e < 2; ++e) {
+                if (8 * j + 2 * q + e < nbk) {
+                    if (r_up < n) out[e * e_col] = (S)X[e];
+                    if (r_lo < n) out[e * e_col + e_row] = (S)X[2 + e];
+                }
             }
+            out += e_step;
+            if (cnt >= 1) strip_update<1, 5>(C, X, tile);
+            if (cnt >= 6) strip_update<6, 5>(C, X, tile);
+            if (cnt >= 11) strip_update<11, 5>(C, X, tile);
         }
-        out += e_step;
-        if (cnt >= 1) strip_update<1, 5>(C, X, tile);
-        if (cnt >= 6) strip_update<6, 5>(C, X, tile);
-        if (cnt >= 11) strip_update<11, 5>(C, X, tile);
-    }
+    };
+    // (two loops: with the choice in the loop the panels of n = 2048 took 2 us longer each)
+    if (any_nonfinite(C)) run(std::true_type{});
+    else run(std::false_type{});
 }
 
 template <class S, bool UP>

@@ -30,6 +30,7 @@
 #include "common.cuh"
 #include "ddla_kernels_internal.h"
 #include "profile.h"
+#include "tile8.cuh"
 
 namespace ddlak {
 
@@ -605,21 +606,29 @@ __global__ void __launch_bounds__(NT, 2) k_potrs_dmma(const TL* __restrict__ A, 
         return make_double2(p[0], p[p1 ? PD_LD : 1]);
     };
     const double2 va = off(ta, ta), vb = off(tb, tb), vab = off(tb, ta);  // (inverses on the diagonal)
+    bool odd = false;  // NaN or infinities among the right-hand sides
     {
         double* p = Xs + row * PD_LDX + 8 * (warp >> 2) + 2 * q;
-        p[0] = acc[0] + acc2[0];
-        p[1] = acc[1] + acc2[1];
-        p[8 * PD_LDX] = acc[2] + acc2[2];
-        p[8 * PD_LDX + 1] = acc[3] + acc2[3];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const double c = acc[i] + acc2[i];
+            p[8 * (i >> 1) * PD_LDX + (i & 1)] = c;
+            odd |= (__double2hiint(c) & 0x7ff00000) == 0x7ff00000;
+        }
     }
-    __syncthreads();
+    odd = __syncthreads_or(odd);
     if (mine) {
         const double* xa = Xs + (8 * ta + 2 * q) * PD_LDX + 8 * h + g;
         const double* xb = Xs + (8 * tb + 2 * q) * PD_LDX + 8 * h + g;
         double Ca[2] = {xa[0], xa[PD_LDX]}, Cb[2] = {xb[0], xb[PD_LDX]};
         double Xa[2] = {0.0, 0.0}, Xb[2] = {0.0, 0.0};
         double* xt = Xt + h * PD_XT + 2 * lane;
-        auto solve = [&](const double (&C)[2], double2 v, double (&X)[2]) {
+        auto solve = [&](const double (&C)[2], int j, double2 v, double (&X)[2]) {
+            if (odd) {
+                const double2 x = tri_row(C[0], C[1], Db + 8 * j * (PD_LD + 1), p1 ? PD_LD : 1, p1 ? 1 : PD_LD, fwd, lane);
+                X[0] = x.x, X[1] = x.y;
+                return;
+            }
             X[0] = X[1] = 0.0;
             pd_mma8(X, C[0], v.x);
             pd_mma8(X, C[1], v.y);
@@ -634,9 +643,9 @@ __global__ void __launch_bounds__(NT, 2) k_potrs_dmma(const TL* __restrict__ A, 
             const int ja = 2 * jb + (fwd ? 0 : 1), jc = 2 * jb + (fwd ? 1 : 0);
             double2 o[4];
             if (w == jb) {
-                solve(Ca, va, Xa);
+                solve(Ca, ta, va, Xa);
                 update(Cb, Xa[0], Xa[1], vab);
-                solve(Cb, vb, Xb);
+                solve(Cb, tb, vb, Xb);
                 if (s + 1 < RB / 16) {
                     *reinterpret_cast<double2*>(xt + ta * 64) = make_double2(Xa[0], Xa[1]);
                     *reinterpret_cast<double2*>(xt + tb * 64) = make_double2(Xb[0], Xb[1]);

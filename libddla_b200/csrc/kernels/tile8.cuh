@@ -5,6 +5,41 @@
 
 namespace ddlak {
 
+// Is an entry of the N tiles NaN or infinite, in any lane of the warp?  (integer pipe)
+template <int N>
+__device__ __forceinline__ bool any_nonfinite(const double (&C)[N][4])
+{
+    constexpr int e = 0x7ff00000;
+    bool odd = false;
+#pragma unroll
+    for (int l = 0; l < N; ++l)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) odd |= (__double2hiint(C[l][i]) & e) == e;
+    return __any_sync(0xffffffffu, odd);
+}
+
+// One row of X = C M for an 8 x 8 triangular M, M(m, c) = mat[m * sm + c * sc] zero for m > c
+// (low) or m < c, without its zeros' products: an infinite or NaN entry of C reaches
+// the columns it belongs to and no others, as in substitution.  For rows that hold one;
+// the others take the tensor-core product of the whole tile.  Lanes 4g .. 4g + 3 hold row g,
+// lane q of them the entries 2q and 2q + 1; all lanes of the warp.  Out of line: inlined it cost
+// the batched kernel 4 % (FP32, code size) on matrices that never take it.
+static __device__ __noinline__ double2 tri_row(double c0, double c1, const double* mat, int sm, int sc, bool low, int lane)
+{
+    double x[2] = {0.0, 0.0};
+#pragma unroll 1
+    for (int m = 0; m < 8; ++m) {
+        const int src = (lane & ~3) | (m >> 1);
+        const double u = __shfl_sync(0xffffffffu, c0, src), v = __shfl_sync(0xffffffffu, c1, src);
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const int c = 2 * (lane & 3) + e;
+            if (low ? m <= c : m >= c) x[e] = fma(m & 1 ? v : u, mat[m * sm + c * sc], x[e]);
+        }
+    }
+    return make_double2(x[0], x[1]);
+}
+
 // T: the tile in shared memory, row-major, lower part.  Its first kv columns are factored,
 // redundantly in every lane (a column costs one reciprocal square root, a multiply and a
 // multiply-add, no shuffles; lane c carries column c of the inverse along): L into Lt

@@ -34,6 +34,8 @@
 // a failed matrix keeps its right-hand side and gets logdet NaN.
 #include <cuda_runtime.h>
 
+#include <type_traits>
+
 #include <ddla_kernels.h>
 
 #include "common.cuh"
@@ -207,11 +209,16 @@ __device__ void vb_matrix(int n, T* __restrict__ A, long long lda, T* __restrict
             cp_group_wait<0>();
 
             // one step of a strip: X = C_0 Inv^T, its columns before `good` stored; then the update
-            auto solve_step = [&](int j, double (&X)[4]) {
+            auto solve_step = [&](int j, auto odd, double (&X)[4]) {
                 const double2 v = *reinterpret_cast<const double2*>(&Inv[j * 64 + g * 8 + 2 * q]);
                 X[0] = X[1] = X[2] = X[3] = 0.0;
                 vb_mma(X, C[0][0], C[0][2], v.x);
                 vb_mma(X, C[0][1], C[0][3], v.y);
+                if (odd) {
+                    const double2 u = tri_row(C[0][0], C[0][1], Inv + j * 64, 1, 8, true, lane);
+                    const double2 l = tri_row(C[0][2], C[0][3], Inv + j * 64, 1, 8, true, lane);
+                    X[0] = u.x, X[1] = u.y, X[2] = l.x, X[3] = l.y;
+                }
             };
             auto store = [&](int j, const double (&X)[4], int rmin, int good) {
 #pragma unroll
@@ -258,6 +265,7 @@ __device__ void vb_matrix(int n, T* __restrict__ A, long long lda, T* __restrict
                         __syncwarp();
                     }
                 } else if (warp < DW) {
+                    const bool odd = any_nonfinite(C);
 #pragma unroll 1
                     for (int j = 0; j < steps; ++j) {
                         const int kv = min(8, nw - 8 * j);
@@ -269,7 +277,7 @@ __device__ void vb_matrix(int n, T* __restrict__ A, long long lda, T* __restrict
                         asm volatile("bar.sync 2, %0;" ::"n"(32 * (DW + 1)) : "memory");
                         const int fl = s_flag[0];
                         double X[4];
-                        solve_step(j, X);
+                        solve_step(j, odd || fl != 0, X);
                         *reinterpret_cast<double2*>(&Xs[(j * W + r_up - J) * 8 + 2 * q]) = make_double2(X[0], X[1]);
                         *reinterpret_cast<double2*>(&Xs[(j * W + r_lo - J) * 8 + 2 * q]) = make_double2(X[2], X[3]);
                         asm volatile("bar.sync 4, %0;" ::"n"(32 * DW) : "memory");
@@ -281,16 +289,20 @@ __device__ void vb_matrix(int n, T* __restrict__ A, long long lda, T* __restrict
                 __syncthreads();  // the block, its inverses and the flag are published
                 info = s_flag[0];
             } else if (active) {
+                auto run = [&](auto odd) {
 #pragma unroll 1
-                for (int j = 0; j < steps; ++j) {
-                    const int good = info ? info - 1 - J - 8 * j : nw - 8 * j;  // final columns from here
-                    if (good <= 0) break;
-                    double X[4];
-                    solve_step(j, X);
-                    store(j, X, 0, min(good, 8));
-                    if (info && good < 8) break;
-                    update(j, RT - 1 - j, X);
-                }
+                    for (int j = 0; j < steps; ++j) {
+                        const int good = info ? info - 1 - J - 8 * j : nw - 8 * j;  // final columns from here
+                        if (good <= 0) break;
+                        double X[4];
+                        solve_step(j, odd, X);
+                        store(j, X, 0, min(good, 8));
+                        if (info && good < 8) break;
+                        update(j, RT - 1 - j, X);
+                    }
+                };
+                // (a failed pivot may have put NaN in its column of every row)
+                run(info || any_nonfinite(C));
             }
         }
         __syncthreads();  // the block column is in A

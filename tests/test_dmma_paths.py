@@ -178,6 +178,120 @@ def test_solve_is_backward_stable(handle, uplo, side, n, noise):
 
 
 @pytest.mark.parametrize("p", ["s", "d"])
+@pytest.mark.parametrize("uplo", ["L", "U"])
+@pytest.mark.parametrize("value", [np.nan, np.inf])
+@pytest.mark.parametrize("r,c", [(5, 2), (14, 3), (100, 50), (127, 126), (128, 5), (190, 63)])
+def test_entries_that_are_not_finite_stay_behind_their_column(handle, p, uplo, value, r, c):
+    """A NaN or infinite entry (r, c) fails the pivot of row r; what substitution computes before it,
+    row r's columns before c among them, is what it is without the entry."""
+    n = 200
+    a = spd(n, 3).astype(NP[p]).astype(np.float64)
+    want = np.linalg.cholesky(a)
+    b = a.copy()
+    b[r, c] = b[c, r] = value
+    t, ptr = device(b, n + 1, p)
+    assert potrf(handle, p, uplo, n, ptr, n + 1) == r + 1
+    out = host(t, n, n, n + 1).astype(np.float64)
+    low = np.tril(out) if uplo == "L" else np.triu(out).T
+    tol = 50 * n * EPS[p]
+    assert np.allclose(low[r, :c], want[r, :c], rtol=0, atol=tol)
+    assert not np.isfinite(low[r, c])
+    # the other rows of the blocks that were finished, and of the failed block
+    rows = np.array([i for i in range(n if r >= 128 else 128) if i != r])
+    cols = 128 if r >= 128 else r
+    keep = rows[:, None] >= np.arange(cols)[None]
+    assert np.allclose(low[rows][:, :cols][keep], want[rows][:, :cols][keep], rtol=0, atol=tol)
+
+
+@pytest.mark.parametrize("p", ["s", "d"])
+@pytest.mark.parametrize("uplo", ["L", "U"])
+@pytest.mark.parametrize("side", ["L", "R"])
+@pytest.mark.parametrize("row", [0, 6, 33, 63, 64, 77, 129])
+def test_forward_solve_leaves_the_rows_before_a_nan(handle, p, uplo, side, row):
+    torch = _torch()
+    from libddla_b200.ddla import _c_api as C
+
+    n, nrhs = 130, 11
+    a = spd(n, 4)
+    low = np.linalg.cholesky(a).astype(NP[p])
+    b = np.random.default_rng(row).standard_normal((n, nrhs)).astype(NP[p])
+    want = np.linalg.solve(low.astype(np.float64), b.astype(np.float64))
+    b[row, 9] = np.nan
+    b[row, 2] = np.inf
+    ta, pa = device(low if uplo == "L" else low.T, n + 1, p)
+    tb, pb = device(b if side == "L" else b.T, n if side == "L" else nrhs, p)
+    C.lib.ddlak_potrs_workspace.restype = ctypes.c_ulonglong
+    work = torch.zeros(int(C.lib.ddlak_potrs_workspace(n, nrhs)), dtype=torch.uint8, device="cuda")
+    f = C.lib.ddlak_forward_solve
+    f.restype = ctypes.c_int
+    f.argtypes = ([ctypes.c_char] * 3 + [ctypes.c_int] * 2 +
+                  [ctypes.c_void_p, ctypes.c_longlong, ctypes.c_void_p, ctypes.c_longlong, ctypes.c_void_p,
+                   ctypes.c_ulonglong, ctypes.c_void_p])
+    torch.cuda.synchronize()
+    assert f(p.encode(), uplo.encode(), side.encode(), n, nrhs, pa, n + 1, pb, n if side == "L" else nrhs,
+             work.data_ptr(), work.numel(), torch.cuda.current_stream().cuda_stream) == 0
+    torch.cuda.synchronize()
+    x = host(tb, n, nrhs, n) if side == "L" else host(tb, nrhs, n, nrhs).T
+    tol = 50 * n * EPS[p] * np.max(np.abs(want))
+    whole = [k for k in range(nrhs) if k not in (2, 9)]
+    assert np.allclose(x[:, whole], want[:, whole], rtol=0, atol=tol)
+    assert np.allclose(x[:row, [2, 9]], want[:row, [2, 9]], rtol=0, atol=tol)
+    assert not np.any(np.isfinite(x[row, [2, 9]]))
+
+
+def batched_run(p, variant, mats, ldas, shifts, rhs):
+    """ddlak_posv_vbatched with one variant for all: (factors, solutions, info, logdet); rhs None: no solve."""
+    torch = _torch()
+    from libddla_b200.ddla import _c_api as C
+
+    up = lambda v, dt: torch.tensor(np.array(v, dtype=dt), device="cuda")  # noqa: E731
+    count, orders = len(mats), [m.shape[0] for m in mats]
+    ta = [device(m, lda, p, s) for m, lda, s in zip(mats, ldas, shifts)]
+    tb = [device(b, b.shape[0], p) for b in rhs] if rhs is not None else []
+    dn, dl, da = up(orders, np.int32), up(ldas, np.int32), up([x[1] for x in ta], np.int64)
+    db = up([x[1] for x in tb], np.int64) if rhs is not None else None
+    logdet = torch.zeros(count, dtype=torch.float64, device="cuda")
+    info = torch.full((count,), -5, dtype=torch.int32, device="cuda")
+    sel = torch.full((count,), variant, dtype=torch.uint8, device="cuda")
+    counters = torch.zeros(2, dtype=torch.int32, device="cuda")
+    f = C.lib.ddlak_posv_vbatched
+    f.restype = ctypes.c_int
+    f.argtypes = [ctypes.c_char, ctypes.c_int, ctypes.c_int] + [ctypes.c_void_p] * 9 + [ctypes.c_int, ctypes.c_void_p]
+    torch.cuda.synchronize()
+    rc = f(p.encode(), 512, count, dn.data_ptr(), da.data_ptr(), dl.data_ptr(), db.data_ptr() if db is not None else None,
+           logdet.data_ptr(), info.data_ptr(), None, sel.data_ptr(), counters.data_ptr(), 7,
+           torch.cuda.current_stream().cuda_stream)
+    assert rc == 0
+    torch.cuda.synchronize()
+    outs = [host(t, n, n, lda, s).astype(np.float64) for (t, _), n, lda, s in zip(ta, orders, ldas, shifts)]
+    xs = [host(t, n, 1, n).astype(np.float64) for (t, _), n in zip(tb, orders)]
+    return outs, xs, info.cpu().numpy(), logdet.cpu().numpy()
+
+
+@pytest.mark.parametrize("p", ["s", "d"])
+@pytest.mark.parametrize("variant", [0, 1])
+@pytest.mark.parametrize("value", [np.nan, np.inf])
+def test_batched_entries_that_are_not_finite(handle, p, variant, value):
+    """As above for the batched kernel: inside the diagonal block, below it, in a later round of rows."""
+    n = 230
+    places = [(5, 2), (20, 11), (40, 5), (63, 62), (100, 45), (200, 70), (229, 30)]
+    a = [spd(n, 31 + i).astype(NP[p]).astype(np.float64) for i in range(len(places))]
+    bad = [m.copy() for m in a]
+    for m, (r, c) in zip(bad, places):
+        m[r, c] = m[c, r] = value
+    outs, xs, info, logdet = batched_run(p, variant, bad, [n + 1] * len(a), [0] * len(a), [np.ones((n, 1))] * len(a))
+    width = (32, 64)[variant]
+    for i, (r, c) in enumerate(places):
+        assert info[i] == r + 1 and np.isnan(logdet[i]) and np.all(xs[i] == 1.0)
+        low, want = np.tril(outs[i]), np.linalg.cholesky(a[i])
+        tol = 50 * n * EPS[p]
+        assert np.allclose(low[r, :c], want[r, :c], rtol=0, atol=tol) and not np.isfinite(low[r, c])
+        done = r // width * width  # the block columns before the failed one are finished
+        rows = np.arange(n) != r
+        assert np.allclose(low[rows][:, :done], np.tril(want)[rows][:, :done], rtol=0, atol=tol)
+
+
+@pytest.mark.parametrize("p", ["s", "d"])
 @pytest.mark.parametrize("variant", [0, 1])
 @pytest.mark.parametrize("solve", [False, True])
 def test_batched_variants(handle, p, variant, solve):
