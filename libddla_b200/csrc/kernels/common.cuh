@@ -105,7 +105,8 @@ __device__ __forceinline__ void lview_st(T* A, long long lda, long long i, long 
     else A[i + j * lda] = v;
 }
 
-// 1/d for positive normal pivots: the hardware's approximate reciprocal
+// 1/d for positive normal pivots (not for subnormal or infinite ones: callers that can meet those
+// look for them, tile8.cuh and panel.cu): the hardware's approximate reciprocal
 // (rcp.approx.ftz.f64, about single precision) refined by two Newton-Raphson
 // steps r <- r + r (1 - d r), each of which squares the relative error, so the
 // result is within an ulp or two of 1/d (a non-positive pivot stops the factorization
@@ -121,8 +122,8 @@ __device__ __forceinline__ double recip_pivot(double d)
 }
 __device__ __forceinline__ float recip_pivot(float d) { return 1.0f / d; }
 
-// 1/sqrt(d) for a positive normal d: the hardware's approximation (about 20 bits)
-// and one step of Householder's third-order iteration for y^-2 = d,
+// 1/sqrt(d) for a positive normal d (NaN or infinite where d is subnormal or infinite):
+// the hardware's approximation (about 20 bits) and one step of Householder's third-order iteration for y^-2 = d,
 // y <- y + y (e/2 + 3 e^2/8), e = 1 - d y^2, which cubes the relative error.
 __device__ __forceinline__ double rsqrt_pivot(double d)
 {

@@ -319,7 +319,10 @@ __global__ void __launch_bounds__(TR_NT) k_trsm_panel_dmma(S* __restrict__ A, lo
     if constexpr (std::is_same<S, double>::value) cp_group_wait<0>();
     __syncthreads();
     // the reciprocal pivots, one a thread (rows at or past nbk: the identity)
-    Rp[t] = t < nbk ? recip_pivot(Lt[tr_tile(t >> 3, t >> 3) + tr_elem(t & 7, t & 7)]) : 1.0;
+    {
+        const double l = t < nbk ? Lt[tr_tile(t >> 3, t >> 3) + tr_elem(t & 7, t & 7)] : 1.0;
+        Rp[t] = isinf(l) ? 0.0 : recip_pivot(l);  // (the square root of a positive double is normal)
+    }
     __syncthreads();
     {
         // column c of tile b's inverse: L y = e_c

@@ -40,6 +40,43 @@ static __device__ __noinline__ double2 tri_row(double c0, double c1, const doubl
     return make_double2(x[0], x[1]);
 }
 
+// factor_tile8 for a tile with a pivot that is subnormal or infinite, outside the range of
+// rsqrt_pivot: by CUDA's square root and division, lane 0 the factor, lane c column c of the
+// inverse.
+static __device__ __noinline__ int factor_tile8_wide(const double* T, double* Inv, double* Lt, double* rinv, int kv,
+                                                     int lane)
+{
+    int good = kv;
+    if (lane == 0) {
+        for (int e = 0; e < 64; ++e) Lt[e] = (e & 7) <= (e >> 3) ? T[e] : 0.0;
+        for (int k = 0; k < kv; ++k) {
+            const double d = Lt[k * 9];
+            if (!(d > 0.0)) {
+                good = k;
+                break;
+            }
+            const double s = sqrt(d);
+            Lt[k * 9] = s;
+            for (int i = k + 1; i < 8; ++i) Lt[i * 8 + k] /= s;
+            for (int i = k + 1; i < 8; ++i)
+                for (int m = k + 1; m <= i && m < kv; ++m) Lt[i * 8 + m] -= Lt[i * 8 + k] * Lt[m * 8 + k];
+        }
+    }
+    good = __shfl_sync(0xffffffffu, good, 0);
+    __syncwarp();
+    if (lane < 8) {
+        for (int i = 0; i < 8; ++i) {
+            double s = i == lane ? 1.0 : 0.0;
+            if (i < good)
+                for (int k = lane; k < i; ++k) s -= Lt[i * 8 + k] * Inv[k * 8 + lane];
+            Inv[i * 8 + lane] = i >= lane && i < good ? s / Lt[i * 9] : 0.0;
+        }
+        if (rinv != nullptr && lane < good) rinv[lane] = 1.0 / Lt[lane * 9];
+    }
+    __syncwarp();
+    return good;
+}
+
 // T: the tile in shared memory, row-major, lower part.  Its first kv columns are factored,
 // redundantly in every lane (a column costs one reciprocal square root, a multiply and a
 // multiply-add, no shuffles; lane c carries column c of the inverse along): L into Lt
@@ -108,6 +145,10 @@ __device__ __forceinline__ int factor_tile8(const double* T, double* Inv, double
         for (int h = 0; h <= r / 2; ++h)
             *reinterpret_cast<double2*>(&Lt[r * 8 + 2 * h]) = make_double2(a[r][2 * h], 2 * h + 1 <= r ? a[r][2 * h + 1] : 0.0);
     __syncwarp();
+    // once more where a pivot was subnormal or infinite: its reciprocal root is NaN or infinite then
+    // (asked here, behind the stores, which hide behind the chain of pivots)
+    if (__any_sync(0xffffffffu, (__double2hiint(rk) & 0x7ff00000) == 0x7ff00000))
+        good = factor_tile8_wide(T, Inv, Lt, rinv, kv, lane);
     return good;
 }
 

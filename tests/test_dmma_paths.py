@@ -291,6 +291,64 @@ def test_batched_entries_that_are_not_finite(handle, p, variant, value):
         assert np.allclose(low[rows][:, :done], np.tril(want)[rows][:, :done], rtol=0, atol=tol)
 
 
+@pytest.mark.parametrize("variant", [0, 1])
+def test_pivot_helpers_over_the_exponent_range(handle, variant):
+    """sqrt(d) and b / sqrt(d) of a tile, against correctly rounded ones: d from the smallest subnormal
+    to the largest double, powers of two and values between.  2 u for the root (one rounding after the
+    correction), 4 u for the quotient (reciprocal root and product)."""
+    rng = np.random.default_rng(9)
+    exps = np.unique(np.concatenate([np.arange(-1074, -1000, 7), np.arange(-1074, 1024, 61), [-1023, -1022, -1021, 1023]]))
+    d = np.ldexp(1.0, exps)
+    d = np.concatenate([d, [v for v in d * rng.uniform(1, 2, d.size) if np.isfinite(v)], [np.finfo(np.float64).max]])
+    # b = 0.75 sqrt(d), the last pivot 1 - 0.75^2
+    mats = [np.array([[v, 0.75 * np.sqrt(v)], [0.75 * np.sqrt(v), 1.0]]) for v in d] + [np.array([[v]]) for v in d]
+    outs, _, info, logdet = batched_run("d", variant, mats, [m.shape[0] for m in mats], [0] * len(mats), None)
+    assert np.all(info == 0) and np.all(np.isfinite(logdet))
+    u = EPS["d"] / 2
+    for m, out in zip(mats, outs):
+        root = np.sqrt(m[0, 0])
+        assert abs(out[0, 0] - root) <= 2 * u * root
+        if m.shape[0] == 2:
+            assert abs(out[1, 0] - m[1, 0] / root) <= 4 * u * 0.75
+
+
+@pytest.mark.parametrize("uplo", ["L", "U"])
+def test_panel_over_the_exponent_range(handle, uplo):
+    """A diagonal block of pivots from 1e-320 to 1e300, one row below it: b / sqrt(d) within 6 u."""
+    n = 129
+    d = 10.0 ** np.random.default_rng(2).permutation(np.linspace(-320, 300, 128))
+    a = np.diag(np.append(d, 1.0))
+    a[128, :128] = a[:128, 128] = np.sqrt(d) / 16
+    t, ptr = device(a, n, "d")
+    assert potrf(handle, "d", uplo, n, ptr, n) == 0
+    out = host(t, n, n, n)
+    low = np.tril(out) if uplo == "L" else np.triu(out).T
+    u = EPS["d"] / 2
+    assert np.all(np.abs(np.diag(low)[:128] - np.sqrt(d)) <= 2 * u * np.sqrt(d))
+    want = a[128, :128] / np.sqrt(d)
+    assert np.all(np.abs(low[128, :128] - want) <= 6 * u * want)
+
+
+@pytest.mark.parametrize("p", ["s", "d"])
+@pytest.mark.parametrize("uplo", ["L", "U"])
+@pytest.mark.parametrize("k", [0, 7, 100, 127, 150, 199])
+def test_infinite_pivot(handle, p, uplo, k):
+    """As sqrt and division give it: an infinite diagonal entry, zeros below it, the rest as without
+    that row and column."""
+    n = 200
+    a = spd(n, 6).astype(NP[p]).astype(np.float64)
+    b = a.copy()
+    b[k, k] = np.inf
+    t, ptr = device(b, n, p)
+    assert potrf(handle, p, uplo, n, ptr, n) == 0
+    out = host(t, n, n, n).astype(np.float64)
+    low = np.tril(out) if uplo == "L" else np.triu(out).T
+    assert low[k, k] == np.inf and np.all(low[k + 1:, k] == 0)
+    rest = np.delete(np.arange(n), k)
+    want = np.linalg.cholesky(a[np.ix_(rest, rest)])
+    assert np.allclose(low[np.ix_(rest, rest)], want, rtol=0, atol=50 * n * EPS[p])
+
+
 @pytest.mark.parametrize("p", ["s", "d"])
 @pytest.mark.parametrize("variant", [0, 1])
 @pytest.mark.parametrize("solve", [False, True])
