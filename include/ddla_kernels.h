@@ -288,9 +288,8 @@ int ddlak_scale_cols(const void* x, void* y, int n, int ncol, double alpha, cons
 
 /* ---- batched uneven Cholesky (ddla::posvVbatched; no reference counterpart) ---- */
 
-/* The labels of the kernel's two per-matrix variants (widths[2]) for type 's'/'d' and
- * kernel instance nmax (512 or 1024), as tuning reports name them; the block columns
- * behind them are 32 and 64 columns wide. */
+/* Block-column widths of the kernel's two per-matrix variants (widths[2]) for type
+ * 's'/'d' and kernel instance nmax (512 or 1024). */
 int ddlak_vbatched_variants(char type, int nmax, int* widths);
 
 /* SMs x resident CTAs of the persistent kernel on the current device (0 on error). */

@@ -469,12 +469,9 @@ extern "C" int ddlak_vbatched_variants(char type, int nmax, int* widths)
 {
     if (nmax != 512 && nmax != 1024) return (int)cudaErrorInvalidValue;
     using namespace ddlak;
-    // The labels a tuning report names the two variants by, per type and instance; the block
-    // columns behind them are VbWidths::w0 = 32 and w1 = 64 columns wide for all.
     if (type != 'd' && type != 's') return (int)cudaErrorInvalidValue;
-    const bool wide = type == 's' && nmax == 512;
-    widths[0] = wide ? 16 : 8;
-    widths[1] = wide ? 32 : 16;
+    widths[0] = VbWidths::w0;
+    widths[1] = VbWidths::w1;
     return 0;
 }
 

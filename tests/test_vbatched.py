@@ -186,7 +186,7 @@ def test_vbatched_autotune_and_tune_file(handle, tmp_path):
     and a fresh process loads it."""
     from libddla_b200.ddla import batched
     t0 = batched.tuning(handle, "d", 512)
-    assert t0["grid"] > 0 and t0["widths"] == [8, 16]
+    assert t0["grid"] > 0 and t0["widths"] == [32, 64]
     path = tmp_path / "vb.tune"
     code = (
         "import json, sys; sys.path.insert(0, '.');"
