@@ -62,7 +62,8 @@ private:
 // the fastest choices are kept per (device, type, max_n bucket) and used by
 // every later posvVbatched / VbatchedPlan.  When the environment variable
 // DDLA_VBATCHED_TUNE_FILE names a file, tables are loaded from it on first use
-// and written back after tuning.  type is 's' or 'd'.
+// and written back after tuning; a table that names other block-column widths than
+// the kernel's (or none) is ignored.  type is 's' or 'd'.
 void vbatchedAutotune(const DdlaHandle_t& handle, char type, int max_n);
 
 struct VbatchedTuning {

@@ -11,10 +11,12 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <fstream>
 #include <map>
 #include <memory>
 #include <mutex>
 #include <numeric>
+#include <sstream>
 #include <stdexcept>
 #include <string>
 #include <tuple>
@@ -58,35 +60,40 @@ bool& tune_file_loaded()
 
 const char* tune_file() { return std::getenv("DDLA_VBATCHED_TUNE_FILE"); }
 
-// File format, one table per line:  <device> <type> <nmax> <grid> <v_0> ... <v_{nmax/16-1}>
+// File format, one table per line:
+//   <device> <type> <nmax> <grid> <width 0> <width 1> <v_0> ... <v_{nmax/16-1}>
+// A line whose widths are not the kernel's was tuned for another kernel and is ignored (so is a
+// line of the older format, without widths: its first choices, 0 or 1, stand in their place).
 void load_tune_file_locked()
 {
     if (tune_file_loaded()) return;
     tune_file_loaded() = true;
     const char* path = tune_file();
     if (!path || !*path) return;
-    FILE* f = std::fopen(path, "r");
-    if (!f) return;
-    int dev, nmax, grid;
-    char type;
-    while (std::fscanf(f, "%d %c %d %d", &dev, &type, &nmax, &grid) == 4) {
-        if ((nmax != 512 && nmax != 1024) || (type != 's' && type != 'd') || grid <= 0) break;
+    std::ifstream f(path);
+    std::string text;
+    while (std::getline(f, text)) {
+        std::istringstream line(text);
+        int dev, nmax, grid, w0, w1;
+        char type;
+        if (!(line >> dev >> type >> nmax >> grid >> w0 >> w1)) continue;
+        if ((nmax != 512 && nmax != 1024) || (type != 's' && type != 'd') || grid <= 0) continue;
         VbatchedTuning tt;
+        ddlak_vbatched_variants(type, nmax, tt.widths);
+        if (w0 != tt.widths[0] || w1 != tt.widths[1]) continue;
         tt.nmax = nmax;
         tt.grid = grid;
         tt.variant.assign(nmax / kBucket, 0);
         bool ok = true;
         for (auto& v : tt.variant) {
             int x;
-            if (std::fscanf(f, "%d", &x) != 1 || x < 0 || x > 1) { ok = false; break; }
+            if (!(line >> x) || x < 0 || x > 1) { ok = false; break; }
             v = (unsigned char)x;
         }
-        if (!ok) break;
-        ddlak_vbatched_variants(type, nmax, tt.widths);
+        if (!ok) continue;
         tt.tuned = true;
         tune_tables()[TuneKey{dev, type, nmax}] = tt;
     }
-    std::fclose(f);
 }
 
 void save_tune_file_locked()
@@ -97,7 +104,8 @@ void save_tune_file_locked()
     if (!f) return;
     for (const auto& kv : tune_tables()) {
         if (!kv.second.tuned) continue;
-        std::fprintf(f, "%d %c %d %d", std::get<0>(kv.first), std::get<1>(kv.first), kv.second.nmax, kv.second.grid);
+        std::fprintf(f, "%d %c %d %d %d %d", std::get<0>(kv.first), std::get<1>(kv.first), kv.second.nmax,
+                     kv.second.grid, kv.second.widths[0], kv.second.widths[1]);
         for (unsigned char v : kv.second.variant) std::fprintf(f, " %d", (int)v);
         std::fprintf(f, "\n");
     }

@@ -212,3 +212,26 @@ def test_vbatched_autotune_and_tune_file(handle, tmp_path):
     assert r.returncode == 0, r.stderr
     out2 = json.loads(r.stdout.strip().splitlines()[-1])
     assert out2["before"]["tuned"] and out2["before"] == out["after"]
+
+
+def test_vbatched_tune_file_of_another_kernel_is_ignored(tmp_path):
+    """Lines without the kernel's block-column widths are not applied; the ones with them are."""
+    import libddla_b200
+
+    path = tmp_path / "vb.tune"
+    choices = " ".join(["1", "0"] * 16)
+    path.write_text(f"0 d 512 5 {choices}\n0 d 1024 7 8 16 {choices} {choices}\nnonsense\n0 s 512 9 32 64 {choices}\n")
+    code = (
+        "import json;"
+        "from libddla_b200 import ddla; from libddla_b200.ddla import batched;"
+        "h = ddla.Handle(ddla.Backend.GPU);"
+        "print(json.dumps([batched.tuning(h, t, n) for t, n in (('d', 512), ('d', 1024), ('s', 512))]))"
+    )
+    env = dict(os.environ, DDLA_VBATCHED_TUNE_FILE=str(path))
+    root = os.path.dirname(os.path.dirname(os.path.abspath(libddla_b200.__file__)))
+    r = subprocess.run([sys.executable, "-c", code], cwd=root, env=env, capture_output=True, text=True, timeout=600)
+    assert r.returncode == 0, r.stderr
+    d512, d1024, s512 = json.loads(r.stdout.strip().splitlines()[-1])
+    assert not d512["tuned"] and d512["grid"] != 5
+    assert not d1024["tuned"] and d1024["grid"] != 7
+    assert s512["tuned"] and s512["grid"] == 9 and s512["variant"] == [1, 0] * 16
