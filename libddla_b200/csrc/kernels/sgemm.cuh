@@ -223,7 +223,7 @@ __device__ __forceinline__ void tile(const CUtensorMap* amap, const CUtensorMap*
             issued = cp + NS + 1;
         }
     }
-    if (!TMA) cp_group_wait<0>();
+    if (!TMA) cp_wait_all();
     ok = __syncthreads_and(ok);
     if (TMA && !ok) {  // copies issued for slices consumed .. issued - 1 may still be in flight
         if (t == 0)

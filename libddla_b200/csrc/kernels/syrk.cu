@@ -233,7 +233,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, Cfg::PER_SM)
             issued = cp + NS + 1;
         }
     }
-    if (!TMA) cp_group_wait<0>();
+    if (!TMA) cp_wait_all();
     ok = __syncthreads_and(ok);
     if (TMA && !ok) {  // copies issued for slices consumed .. issued - 1 may still be in flight
         if (threadIdx.x == 0)
