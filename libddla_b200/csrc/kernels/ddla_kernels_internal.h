@@ -35,8 +35,9 @@ cudaError_t syrk_f32(float* A, long long lda, int k0, int nbk, int n, long long 
                      cudaStream_t st);
 
 // W = L^-1 for one lower FP32 factor of any order; what W holds above its diagonal
-// afterwards is unspecified (sgemm.cu).
-cudaError_t trtri_large_f32(int n, const float* L, long long ldl, float* W, long long ldw, cudaStream_t st);
+// afterwards is unspecified; a wait that gives up leaves NaN in its tile and its code in *status
+// (sgemm.cu).
+cudaError_t trtri_large_f32(int n, const float* L, long long ldl, float* W, long long ldw, int* status, cudaStream_t st);
 
 template <class T, bool UP>
 cudaError_t trailing_update_simt(T* A, long long lda, int k0, int nbk, int n, long long t0, int cols,

@@ -984,6 +984,7 @@ extern "C" int ddlak_trtri_blocked(char type, int n, const void* L, long long ld
     if (type == 'd')
         return (int)potrs_launch<double, false, false, double, true>(
             static_cast<const double*>(L), ldl, static_cast<double*>(W), ldw, n, n, flags, ticket, status, st);
-    if (type == 's') return (int)trtri_large_f32(n, static_cast<const float*>(L), ldl, static_cast<float*>(W), ldw, st);
+    if (type == 's') return (int)trtri_large_f32(n, static_cast<const float*>(L), ldl, static_cast<float*>(W), ldw,
+                                                 status, st);
     return (int)cudaErrorInvalidValue;
 }

@@ -88,7 +88,8 @@ __global__ void __launch_bounds__(sg::NT, UP ? 1 : 2)
 template <int STEP, bool TMA>
 __global__ void __launch_bounds__(sg::NT, 2)
     k_trtri_level_f32(const __grid_constant__ CUtensorMap lmap, const __grid_constant__ CUtensorMap wmap, int n, int h,
-                      int nt, const float* __restrict__ L, long long ldl, float* __restrict__ W, long long ldw)
+                      int nt, const float* __restrict__ L, long long ldl, float* __restrict__ W, long long ldw,
+                      int* status)
 {
     extern __shared__ __align__(128) unsigned char sg_raw[];
     const long long r0 = 2LL * h * blockIdx.y;
@@ -102,7 +103,7 @@ __global__ void __launch_bounds__(sg::NT, 2)
         // T(i, j) = sum_{j0 <= k < h} L21(i, k) W11(k, j); W11(k, j) counts for k >= j
         sg::tile<false, true, TMA, sg::ALL, sg::K_GE_ROW>(&lmap, &wmap, L, ldl, W, ldw, r0 + h + i0, r0 + j0, n, n,
                                                           r0 + j0, (h - j0 + sg::KC - 1) / sg::KC, r0 + h,
-                                                          sg::TILE / sg::KC, 1 << 30, sg_raw, &g_sgemm_status, acc);
+                                                          sg::TILE / sg::KC, 1 << 30, sg_raw, status, acc);
 #pragma unroll
         for (int u = 0; u < 8; ++u)
 #pragma unroll
@@ -115,7 +116,7 @@ __global__ void __launch_bounds__(sg::NT, 2)
         const int kn = min(i0 + sg::TILE, m2);
         sg::tile<false, false, TMA, sg::K_LE_ROW, sg::ALL>(&wmap, &wmap, W, ldw, W, ldw, r0 + h + i0, r0 + j0, n, n,
                                                            r0 + h, (kn + sg::KC - 1) / sg::KC, r0 + h + kn, 0,
-                                                           i0 / sg::KC, sg_raw, &g_sgemm_status, acc);
+                                                           i0 / sg::KC, sg_raw, status, acc);
 #pragma unroll
         for (int v = 0; v < 8; ++v)
 #pragma unroll
@@ -179,7 +180,7 @@ cudaError_t syrk_f32(float* A, long long lda, int k0, int nbk, int n, long long 
 template cudaError_t syrk_f32<false>(float*, long long, int, int, int, long long, int, const int*, cudaStream_t);
 template cudaError_t syrk_f32<true>(float*, long long, int, int, int, long long, int, const int*, cudaStream_t);
 
-cudaError_t trtri_large_f32(int n, const float* L, long long ldl, float* W, long long ldw, cudaStream_t st)
+cudaError_t trtri_large_f32(int n, const float* L, long long ldl, float* W, long long ldw, int* status, cudaStream_t st)
 {
     const int nleaf = (int)ceil_div(n, SL);
     k_trtri_leaf_f32<<<(unsigned)ceil_div(nleaf, 4), 256, 0, st>>>(nleaf, n, L, ldl, W, ldw);
@@ -197,11 +198,11 @@ cudaError_t trtri_large_f32(int n, const float* L, long long ldl, float* W, long
         const int nt = (int)ceil_div(h, sg::TILE);
         const dim3 grid((unsigned)(nt * nt), (unsigned)ceil_div(n - h, 2 * h));
         if (tma) {
-            k_trtri_level_f32<1, true><<<grid, sg::NT, s1, st>>>(lrow, wk, n, h, nt, L, ldl, W, ldw);
-            k_trtri_level_f32<2, true><<<grid, sg::NT, s2, st>>>(lrow, wrow, n, h, nt, L, ldl, W, ldw);
+            k_trtri_level_f32<1, true><<<grid, sg::NT, s1, st>>>(lrow, wk, n, h, nt, L, ldl, W, ldw, status);
+            k_trtri_level_f32<2, true><<<grid, sg::NT, s2, st>>>(lrow, wrow, n, h, nt, L, ldl, W, ldw, status);
         } else {
-            k_trtri_level_f32<1, false><<<grid, sg::NT, s1, st>>>(lrow, wk, n, h, nt, L, ldl, W, ldw);
-            k_trtri_level_f32<2, false><<<grid, sg::NT, s2, st>>>(lrow, wrow, n, h, nt, L, ldl, W, ldw);
+            k_trtri_level_f32<1, false><<<grid, sg::NT, s1, st>>>(lrow, wk, n, h, nt, L, ldl, W, ldw, status);
+            k_trtri_level_f32<2, false><<<grid, sg::NT, s2, st>>>(lrow, wrow, n, h, nt, L, ldl, W, ldw, status);
         }
         note_launches(2);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
