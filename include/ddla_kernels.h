@@ -324,10 +324,11 @@ int ddlak_gp_build(char type, int batch, int n, int d, const void* X, long long 
 int ddlak_trtri_batched(char type, int batch, int n, const void* L, long long ldl, long long lstride, void* W,
                         long long ldw, long long wstride, void* stream);
 
-/* W = L^-1 (lower triangle written; above it W is unspecified) for any n: FP64 by
- * the fused forward substitution of ddlak_potrs on the identity, generated in the
- * kernel, skipping its zero blocks; FP32 by doubling on the FP32 pipe.  Scratch: ddlak_potrs_workspace(n, n);
- * the first int of it is the status word as for ddlak_potrs. */
+/* W = L^-1 (lower triangle written; above it W is unspecified) for any n: by the
+ * fused forward substitution of ddlak_potrs on the identity, generated in the
+ * kernel, skipping its zero blocks; large FP32 factors by doubling on the FP32
+ * pipe.  Scratch: ddlak_potrs_workspace(n, n); the first int of it is the status
+ * word as for ddlak_potrs (nonzero: a wait gave up). */
 int ddlak_trtri_blocked(char type, int n, const void* L, long long ldl, void* W, long long ldw, void* work,
                         unsigned long long work_bytes, void* stream);
 

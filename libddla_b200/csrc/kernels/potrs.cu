@@ -967,8 +967,16 @@ extern "C" int ddlak_forward_solve(char type, char uplo, char side, int n, int n
     }
 }
 
-// W = L^-1 for a lower factor: FP64 by the fused forward substitution on the identity,
-// FP32 by doubling (sgemm.cu).
+// FP32 order from which the inversion is done by doubling (sgemm.cu); below it by the fused
+// substitution on the identity, whose time is n / 64 links where doubling has two launches and
+// a 64-wide serial leaf per level.  us, substitution / doubling, leading dimension n:
+//   n = 200 28 / 130   1025 88 / 674   2048 282 / 616   3600 1183 / 1300   3800 1357 / 1346
+//   4096 1605 / 1393   4100 1678 / 2040   8192 11790 / 5562
+//   odd, without TMA: 5003 2879 / 3079   6001 4733 / 4183   8191 11861 / 7530
+static constexpr int kTrtriDoubling = 3800;
+
+// W = L^-1 for a lower factor: FP64, and FP32 below that order, by the fused forward
+// substitution on the identity, FP32 from there by doubling (sgemm.cu).
 extern "C" int ddlak_trtri_blocked(char type, int n, const void* L, long long ldl, void* W, long long ldw, void* work,
                                    unsigned long long work_bytes, void* stream)
 {
@@ -984,6 +992,9 @@ extern "C" int ddlak_trtri_blocked(char type, int n, const void* L, long long ld
     if (type == 'd')
         return (int)potrs_launch<double, false, false, double, true>(
             static_cast<const double*>(L), ldl, static_cast<double*>(W), ldw, n, n, flags, ticket, status, st);
+    if (type == 's' && n < kTrtriDoubling)
+        return (int)potrs_launch<float, false, false, float, true>(
+            static_cast<const float*>(L), ldl, static_cast<float*>(W), ldw, n, n, flags, ticket, status, st);
     if (type == 's') return (int)trtri_large_f32(n, static_cast<const float*>(L), ldl, static_cast<float*>(W), ldw,
                                                  status, st);
     return (int)cudaErrorInvalidValue;

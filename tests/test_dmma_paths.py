@@ -412,10 +412,39 @@ def test_batched_variants(handle, p, variant, solve):
             assert np.max(np.abs(res)) <= 40 * (n + 1) * EPS[p] * np.linalg.norm(mats[i], 2) * np.max(np.abs(x))
 
 
-@pytest.mark.parametrize("n", [1025, 1101, 1536])
+@pytest.mark.parametrize("p,n", [("s", 1), ("s", 65), ("s", 1025), ("s", 3799), ("s", 3800), ("s", 3801), ("s", 4097),
+                                 ("d", 1), ("d", 65), ("d", 1025)])
+def test_inverse_of_a_large_factor(handle, p, n):
+    """Both sides of the order from which FP32 inverts by doubling, leading dimensions with TMA and
+    without, a last leaf of one row.  Substitution and products alike give |L W - I| <= c n u |L||W|
+    with c a small constant (Higham, section 14.2); 4 here."""
+    torch = _torch()
+    from libddla_b200.ddla import _c_api as C
+
+    dt = torch.float32 if p == "s" else torch.float64
+    g = torch.randn(n, n, device="cuda", dtype=torch.float64, generator=torch.Generator(device="cuda").manual_seed(n))
+    low = torch.linalg.cholesky(g @ g.T / n + torch.eye(n, device="cuda", dtype=torch.float64)).to(dt)
+    store, w = low.T.contiguous(), torch.full((n, n), float("nan"), device="cuda", dtype=dt)
+    C.lib.ddlak_potrs_workspace.restype = ctypes.c_ulonglong
+    work = torch.zeros(int(C.lib.ddlak_potrs_workspace(n, n)), dtype=torch.uint8, device="cuda")
+    f = C.lib.ddlak_trtri_blocked
+    f.restype = ctypes.c_int
+    f.argtypes = [ctypes.c_char, ctypes.c_int, ctypes.c_void_p, ctypes.c_longlong, ctypes.c_void_p, ctypes.c_longlong,
+                  ctypes.c_void_p, ctypes.c_ulonglong, ctypes.c_void_p]
+    assert f(p.encode(), n, store.data_ptr(), n, w.data_ptr(), n, work.data_ptr(), work.numel(),
+             torch.cuda.current_stream().cuda_stream) == 0
+    torch.cuda.synchronize()
+    assert int(work[:4].view(torch.int32)[0]) == 0
+    inv = torch.tril(w.T).double()
+    low = low.double()
+    res = (low @ inv - torch.eye(n, device="cuda", dtype=torch.float64)).abs()
+    bound = 4 * n * EPS[p] / 2 * (low.abs() @ inv.abs())
+    assert bool(torch.all(res <= bound)), float((res / bound).nan_to_num().max())
+
+
+@pytest.mark.parametrize("n", [1025, 1101, 1536, 3801])
 def test_large_fp32_gradient(handle, n):
-    """The FP32 inversion by doubling and the contraction: leading dimensions with TMA (a multiple of
-    4) and without, a last leaf of one row."""
+    """The FP32 inversion and the contraction: leading dimensions with TMA (a multiple of 4) and without."""
     torch = _torch()
     from libddla_b200.ddla import autograd as ag
 
