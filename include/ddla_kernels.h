@@ -207,8 +207,6 @@ int ddlak_potrf_mixed(char precision, int n, void* W, long long ldw, void* P0, v
 int ddlak_potrf_mixed_grouped(char precision, int group, int n, void* W, long long ldw, void* P0, void* P1,
                               int* dinfo, int* status, void* stream);
 
-/* Inverses (FP64) of the 64 x 64 diagonal blocks of an FP32 factor (lower):
- * ddlak_inv_diag_bytes(n) bytes, one column-major block per block row. */
 /* Left-looking mixed factorization fed from host memory: the lower part of A
  * (A_host, leading dimension lda_host) goes to A (device, lda) in column panels
  * of 128 * group columns on copy_stream, and on stream each panel is converted
@@ -222,12 +220,8 @@ int ddlak_potrf_mixed_stream(char precision, int group, int n, const void* A_hos
                              long long lda, void* W, long long ldw, void* Lk, long long ldk, void* colsum, void* anrm,
                              int* dinfo, int* status, void* copy_stream, void* stream);
 
-unsigned long long ddlak_inv_diag_bytes(int n);
-int ddlak_inv_diag_blocks(int n, const void* L32, long long ldl, void* Dinv, void* stream);
-
 /* In-place solve L L^T X = B with an FP32 factor (lower, ldl) and FP64 B;
- * scratch as ddlak_potrs_workspace(n, nrhs).  Dinv (may be NULL) is accepted and
- * not read: the solve inverts its diagonal blocks itself. */
+ * scratch as ddlak_potrs_workspace(n, nrhs).  Dinv is not read (may be NULL). */
 int ddlak_potrs_mixed(int n, int nrhs, const void* L32, long long ldl, const void* Dinv, void* B, long long ldb,
                       void* work, unsigned long long work_bytes, void* stream);
 

@@ -30,7 +30,7 @@ void MixedPreconditioner::apply(double* B, long long ldb) const
     else if (blocked)
         ck(ddlak_bis_solve(n, nrhs, L, ldl, Dinv, B, ldb, work, bytes, h->stream), "preconditioner");
     else
-        ck(ddlak_potrs_mixed(n, nrhs, L, ldl, Dinv, B, ldb, work, bytes, h->stream), "preconditioner");
+        ck(ddlak_potrs_mixed(n, nrhs, L, ldl, nullptr, B, ldb, work, bytes, h->stream), "preconditioner");
 }
 
 GmresIR::GmresIR(const DdlaHandle_t& h, int n, int nrhs, const double* A, long long lda, const MixedPreconditioner& M,

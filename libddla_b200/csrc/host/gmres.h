@@ -18,7 +18,7 @@ namespace ddla {
 // M^-1 = (L L^T)^-1 applied in place to an n x nrhs FP64 block, L the FP32
 // factor: by inverted diagonal super-blocks when `blocked` (FP32 arithmetic
 // with the FP32 inverses Dinv32 when `single`, else FP64 arithmetic), else by
-// the fused chain solve (ddlak_potrs_mixed, which inverts its 64-row diagonal blocks itself).
+// the fused chain solve (ddlak_potrs_mixed).
 struct MixedPreconditioner {
     DdlaHandle_t h = nullptr;
     int n = 0;

@@ -95,11 +95,11 @@ void mixed_core(const DdlaHandle_t& h, char precision, int n, int nrhs, double* 
     const long long ldw = (n + 3) / 4 * 4;
     const std::size_t pbytes = ddlak_mixed_panel_bytes(n);
     // refinement solves: inverted diagonal super-blocks for up to 16 right-hand
-    // sides, the fused chain with 64-row block inverses beyond
+    // sides, the fused chain beyond
     const bool blocked = nrhs <= 16;
     const std::size_t sbytes = blocked ? ddlak_bis_solve_workspace(n, std::max(1, nrhs))
                                        : ddlak_potrs_workspace(n, std::max(1, nrhs));
-    const std::size_t dinv_bytes = blocked ? ddlak_bis_inverse_bytes(n) : ddlak_inv_diag_bytes(n);
+    const std::size_t dinv_bytes = blocked ? ddlak_bis_inverse_bytes(n) : 0;
     const std::size_t dinv32_bytes = blocked ? detail::padded_bytes<float>(ddlak_bis_inverse_bytes(n) / 8) : 0;
     const int kry = GmresIR::kRestart;
     long long ldk = 0;
@@ -123,7 +123,7 @@ void mixed_core(const DdlaHandle_t& h, char precision, int n, int nrhs, double* 
     double* D = detail::take<double>(w, (std::size_t)n * std::max(1, nrhs));
     double* Bc = detail::take<double>(w, (std::size_t)n * std::max(1, nrhs));
     double* colsum = detail::take<double>(w, n);
-    double* Dinv = detail::take<double>(w, dinv_bytes / sizeof(double));
+    double* Dinv = blocked ? detail::take<double>(w, dinv_bytes / sizeof(double)) : nullptr;
     float* Dinv32 = blocked ? detail::take<float>(w, ddlak_bis_inverse_bytes(n) / 8) : nullptr;
     Scalars* sc = detail::take<Scalars>(w, 1);
     double* xn = detail::take<double>(w, std::max(1, nrhs));
@@ -180,7 +180,7 @@ void mixed_core(const DdlaHandle_t& h, char precision, int n, int nrhs, double* 
         detail::DeviceScratch tmp(h, ddlak_bis_inverse_bytes(n));
         ck(ddlak_bis_inverse(n, W, ldw, Dinv, tmp.data(), st), "diagonal block inverses");
         ck(ddlak_bis_inverse_narrow(n, Dinv, Dinv32, st), "FP32 diagonal block inverses");
-    }  // else: the fused solve inverts its diagonal blocks itself
+    }
     MixedPreconditioner M;
     M.h = h;
     M.n = n;

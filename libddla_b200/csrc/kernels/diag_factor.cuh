@@ -49,12 +49,11 @@ constexpr int UP = (MAXN - PW) / 16;  // row groups of the trailing update (6)
 // (A) warp 0: the w x w diagonal block at (c0, c0).  On exit the block's
 // columns before the first failed one hold L, s_rs[c0 + j] = 1 / l_jj for
 // them, and a failure is recorded as *s_fail = c0 + j + 1.
-template <class T, int WC = 0>  // WC: the width when known at compile time (a full panel), else 0
-__device__ __forceinline__ void panel_diag(T* s, int ld, int c0, int w_rt, int lane, T (*colbuf)[PW],
+template <class T>
+__device__ __forceinline__ void panel_diag(T* s, int ld, int c0, int w, int lane, T (*colbuf)[PW],
                                            real_t<T>* s_inv, real_t<T>* s_rs, int* s_fail)
 {
     using R = real_t<T>;
-    const int w = WC ? WC : w_rt;
     const int i = lane;
     T a[PW];
 #pragma unroll

@@ -754,75 +754,10 @@ cudaError_t potrs_dispatch(char type, char uplo, char side, int n, int nrhs, con
 }  // namespace
 }  // namespace ddlak
 
-// ---------------------------------------------------------------------------
-// inverses of the RB x RB diagonal blocks of an FP32 factor, in FP64: one CTA
-// per block, the block widened into shared memory, one thread per column of
-// the inverse (forward substitution against the identity).
-// ---------------------------------------------------------------------------
-namespace ddlak {
-namespace {
-__global__ void __launch_bounds__(128) k_inv_diag_blocks(const float* __restrict__ L, long long ldl, int n,
-                                                         double* __restrict__ Dinv)
-{
-    __shared__ double Ls[RB][RB + 1];  // Ls[c][r] = L(r, c)
-    const int blk = blockIdx.x;
-    const long long i0 = (long long)blk * RB;
-    const int nb = (int)((n - i0) < RB ? (n - i0) : RB);
-    for (int idx = threadIdx.x; idx < RB * RB; idx += blockDim.x) {
-        const int r = idx % RB, c = idx / RB;
-        Ls[c][r] = (r < nb && c < nb && r >= c) ? (double)L[(i0 + r) + (i0 + c) * ldl] : 0.0;
-    }
-    __syncthreads();
-    double* out = Dinv + (long long)blk * RB * RB;
-    const int c = threadIdx.x;
-    if (c < RB) {
-        double y[RB];
-#pragma unroll
-        for (int r = 0; r < RB; ++r) y[r] = 0.0;
-        if (c < nb) {
-#pragma unroll
-            for (int r = 0; r < RB; ++r) {
-                if (r >= c && r < nb) {
-                    double s = r == c ? 1.0 : 0.0;
-#pragma unroll
-                    for (int k = 0; k < RB; ++k)
-                        if (k >= c && k < r) s = fma(-Ls[k][r], y[k], s);
-                    y[r] = s / Ls[r][r];
-                }
-            }
-        }
-#pragma unroll
-        for (int r = 0; r < RB; ++r) out[(long long)c * RB + r] = y[r];
-    }
-}
-}  // namespace
-}  // namespace ddlak
-
-extern "C" unsigned long long ddlak_inv_diag_bytes(int n)
-{
-    return n > 0 ? (unsigned long long)ddlak::ceil_div(n, ddlak::RB) * ddlak::RB * ddlak::RB * sizeof(double) : 0;
-}
-
-extern "C" int ddlak_inv_diag_blocks(int n, const void* L32, long long ldl, void* Dinv, void* stream)
-{
-    using namespace ddlak;
-    if (n <= 0) return 0;
-    const int N = (int)ceil_div(n, RB);
-    {
-        ProfScope ps(PK_MIXED_OTHER, static_cast<cudaStream_t>(stream), (double)N * RB * RB * RB / 3.0,
-                     (double)N * RB * RB * 12.0);
-        k_inv_diag_blocks<<<N, 128, 0, static_cast<cudaStream_t>(stream)>>>(static_cast<const float*>(L32), ldl, n,
-                                                                           static_cast<double*>(Dinv));
-    }
-    note_launches(1);
-    return (int)cudaGetLastError();
-}
-
 // Solve with an FP32 factor (uplo 'L') and FP64 right-hand sides in place
 // (the refinement solves of the mixed-precision path); same scratch as
-// ddlak_potrs.  With Dinv (from ddlak_inv_diag_blocks) the diagonal steps are
-// products with the precomputed inverse blocks instead of substitutions.
-extern "C" int ddlak_potrs_mixed(int n, int nrhs, const void* L32, long long ldl, const void* Dinv, void* B,
+// ddlak_potrs.
+extern "C" int ddlak_potrs_mixed(int n, int nrhs, const void* L32, long long ldl, const void* /*Dinv*/, void* B,
                                  long long ldb, void* work, unsigned long long work_bytes, void* stream)
 {
     using namespace ddlak;
@@ -833,7 +768,6 @@ extern "C" int ddlak_potrs_mixed(int n, int nrhs, const void* L32, long long ldl
     if (e != cudaSuccess) return (int)e;
     int* status = static_cast<int*>(work);
     int* flags = reinterpret_cast<int*>(static_cast<char*>(work) + 256);
-    (void)Dinv;  // accepted; the solve inverts the diagonal blocks itself
     return (int)potrs_launch<double, false, false, float>(static_cast<const float*>(L32), ldl,
                                                           static_cast<double*>(B), ldb, n, nrhs, flags, status + 1,
                                                           status, st);

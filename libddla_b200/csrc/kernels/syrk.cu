@@ -300,8 +300,10 @@ cudaError_t launch_syrk(double* A, long long lda, long long astride, int batch, 
         auto* k = k_syrk_dmma<Cfg, UP, true, BATCH>;
         if ((e = smem_optin(k, smem)) != cudaSuccess) return e;
         k<<<grid, Cfg::THREADS, smem, st>>>(amap, bmap, A, lda, astride, k0, nbk, n, t0, cols, dinfo);
+    } else if constexpr (BATCH) {
+        return cudaErrorInvalidValue;  // its one caller takes even leading dimensions and aligned bases only
     } else {
-        auto* k = k_syrk_dmma<Cfg, UP, false, BATCH>;
+        auto* k = k_syrk_dmma<Cfg, UP, false, false>;
         if ((e = smem_optin(k, smem)) != cudaSuccess) return e;
         k<<<grid, Cfg::THREADS, smem, st>>>(amap, bmap, A, lda, astride, k0, nbk, n, t0, cols, dinfo);
     }
