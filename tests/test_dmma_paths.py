@@ -81,6 +81,39 @@ def test_factor_tile_edges(handle, p, uplo, n):
 
 @pytest.mark.parametrize("p", ["s", "d"])
 @pytest.mark.parametrize("uplo", ["L", "U"])
+@pytest.mark.parametrize("group,n,pad", [(2, 1500, 0), (2, 1501, 0), (4, 1500, 0), (4, 1499, 0), (8, 1500, 2), (8, 1501, 0),
+                                         (1, 2433, 0), (2, 2433, 0), (1, 2432, 0), (4, 2433, 0)])
+def test_super_steps(handle, p, uplo, group, n, pad):
+    """Updates with K up to 1024 (several turns of the stage ring), look-ahead and left-looking regions,
+    and regions of 148 or more 128 x 128 tiles (from n - 128 (1 + group) = 2049), all with and without
+    TMA.  Bound as check_factor's."""
+    torch = _torch()
+    from libddla_b200.ddla import _c_api as C
+
+    g = torch.randn(n, n, device="cuda", dtype=torch.float64, generator=torch.Generator(device="cuda").manual_seed(n))
+    a = (g @ g.T / n + torch.eye(n, device="cuda", dtype=torch.float64)).cpu().numpy().astype(NP[p]).astype(np.float64)
+    a = np.tril(a) + np.tril(a, -1).T
+    lda = n + pad
+    t, ptr = device(a, lda, p)
+    f = C.lib.ddlak_potrf_grouped
+    f.restype = ctypes.c_int
+    f.argtypes = [ctypes.c_char, ctypes.c_char, ctypes.c_int, ctypes.c_int, ctypes.c_void_p, ctypes.c_longlong,
+                  ctypes.c_void_p, ctypes.c_void_p]
+    info = torch.full((1,), -7, dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    assert f(p.encode(), uplo.encode(), group, n, ptr, lda, info.data_ptr(), torch.cuda.current_stream().cuda_stream) == 0
+    torch.cuda.synchronize()
+    assert int(info[0]) == 0
+    out = t.view(n, lda)[:, :n].T
+    low = (torch.tril(out) if uplo == "L" else torch.triu(out).T).double()
+    am = torch.from_numpy(a).cuda()
+    bound = 4 * (n + 1) * EPS[p] * (low.abs() @ low.abs().T) + am.abs() * EPS[p]
+    diff = torch.tril((am - low @ low.T).abs() - bound)
+    assert float(diff.max()) <= 0.0
+
+
+@pytest.mark.parametrize("p", ["s", "d"])
+@pytest.mark.parametrize("uplo", ["L", "U"])
 @pytest.mark.parametrize("bad", [0, 6, 7, 8, 63, 64, 127, 128, 199])
 def test_failed_pivot(handle, p, uplo, bad):
     """info is the failed pivot's order and the columns before it are final."""

@@ -112,3 +112,37 @@ def test_wait_timeout_is_reported_and_handle_recovers(handle):
     ddla.ppotrs(dA, dB, "L")
     X = dB.to_global_matrix()
     assert np.max(np.abs(A @ X - B)) <= 1e-9 * np.max(np.abs(B))
+
+
+@pytest.mark.parametrize("op", ["ppotrs", "pposv"])
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+def test_wait_timeout_of_the_fused_solve(handle, op, dtype):
+    """The solve that runs behind the factorization in one call, and by itself (upper triangle, more
+    right-hand sides than the inverted-block solve takes)."""
+    ddla = _ddla()
+    C = ddla._c_api
+    rng = np.random.default_rng(33)
+    n, nrhs = 2048, 17
+    R = rng.random((n, n))
+    A = (2.0 * np.eye(n) + (R + R.T) / (4 * n)).astype(dtype)
+    B = rng.standard_normal((n, nrhs)).astype(dtype)
+
+    def matrices():
+        return (ddla.DistributedMatrix.from_global_matrix(handle, A, mb=256, nb=256),
+                ddla.DistributedMatrix.from_global_matrix(handle, B, mb=256, nb=256))
+
+    dA, dB = matrices()
+    if op == "ppotrs":
+        assert ddla.ppotrf(dA, "U")[1] == 0
+    assert C.ddla_c_set_wait_budget(handle.ptr, 1) == 0
+    try:
+        with pytest.raises(C.DdlaError, match="timed out"):
+            ddla.ppotrs(dA, dB, "U") if op == "ppotrs" else ddla.pposv(dA, dB, "U")
+    finally:
+        assert C.ddla_c_set_wait_budget(handle.ptr, 0) == 0
+    dA, dB = matrices()
+    _, info = ddla.pposv(dA, dB, "U")
+    assert info == 0
+    X = dB.to_global_matrix().astype(np.float64)
+    tol = 1e-11 if dtype == np.float64 else 1e-3
+    assert np.max(np.abs(A.astype(np.float64) @ X - B)) <= tol * np.max(np.abs(B))
