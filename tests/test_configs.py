@@ -47,6 +47,7 @@ def test_se_kernel_pposv_n16384(handle, p):
     npdt = np.complex128 if cplx else np.float64
     dA = ddla.DistributedMatrix.wrap(handle, Acm.data_ptr(), n, n, n, npdt, mb=256, nb=256)
     dX = ddla.DistributedMatrix.wrap(handle, Xt.data_ptr(), n, nrhs, n, npdt, mb=256, nb=256)
+    torch.cuda.synchronize()  # the handle's stream does not wait for torch's
     _, info = ddla.pposv(dA, dX, "L")
     assert info == 0
     L = torch.tril(Acm.T)
@@ -110,6 +111,7 @@ def test_mixed_pposv_n32768(handle, householder_cases, prec, kappa):
     wrap = lambda t, rows, cols: ddla.DistributedMatrix.wrap(handle, t.data_ptr(), rows, cols, n, np.float64,
                                                             mb=256, nb=256)
     dA, dB, dX = wrap(Acopy, n, n), wrap(Bt, n, nrhs), wrap(Xt, n, nrhs)
+    torch.cuda.synchronize()  # the handle's stream does not wait for torch's
     _, info, rep = ddla.pposv_mixed(dA, dB, dX, precision=prec)
     assert info == 0
     X = Xt.T
