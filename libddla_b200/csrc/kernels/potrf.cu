@@ -19,6 +19,7 @@
 // info follows LAPACK ?potrf: the order of the first leading minor that is not
 // positive definite (diagonal value <= 0 or NaN), 0 on success.  Every kernel
 // returns immediately once info is set, so the first failure is the one kept.
+#include <climits>
 #include <mutex>
 #include <type_traits>
 
@@ -381,18 +382,39 @@ static cudaError_t potrf_enqueue(T* A, long long lda, int n, int G, int* dinfo, 
 
 // Block columns per super-step.  A wide super-step reads and writes the trailing matrix
 // less often, but its left-looking updates (K up to 128 (G - 1) on one block column)
-// lie on the chain, which is all of the time at small orders.  ms with G = 1 / 2 / 4 / 8:
-//   d L  n = 2048 0.86 / 0.91 / 1.0 / 1.1    5003 3.70 / 3.60 / 3.77 / 3.9
-//        8192 - / 8.99 / 8.59 / 8.8          16384 - / - / 52.4 / 50.1
-//   s L  2048 1.56 / 1.57 / 1.74 / 2.15      6000 10.5 / 7.9 / 7.2 / 7.9   16384 184 / 101 / 63 / 49
-//   s U  2048 1.38 / 1.51 / 1.78 / 2.30      6000 6.2 / 6.0 / 6.8 / 8.6    16384 107 / 78 / 65 / 62
-//   c L  2048 3.20 / 3.32 / 3.64 / 4.30      6000 13.6 / 14.3 / 15.5 / 17.9  8192 25.9 / 25.7 / 27.4 / 30.8
-//   z L  2048 2.98 / 3.18 / 3.48 / 4.19      6000 16.5 / 15.4 / 16.1 / 18.4  8192 33.8 / 31.0 / 31.0 / 33.4
-static int potrf_group(char type, int n)
+// lie on the chain, which is all of the time at small orders.  The orders from which 2, 4
+// and 8 are the faster, by type, triangle and, for FP32, whether the update's tiles
+// come by TMA (the cp.async form gains more from a long K).  ms with G = 1 / 2 / 4 / 8, leading dimension n, on both sides of the lines:
+//   d L      3584  1.56 / 1.60 / 1.79 / 2.08    4096  1.98 / 1.98 / 2.18 / 2.65    6144  5.00 / 4.42 / 4.48 / 4.96
+//            7168  7.42 / 6.32 / 6.11 / 6.71    10240 - / 16.2 / 14.7 / 14.7       12288 - / 26.6 / 23.7 / 23.2
+//   d U      1536  .650 / .649 / .709 / .803    4096  2.77 / 2.51 / 2.54 / 2.96    4608  3.64 / 3.23 / 3.13 / 3.43
+//            7168  12.0 / 8.70 / 7.53 / 7.66    8192  17.4 / 12.3 / 10.3 / 10.1    16384 - / 88.8 / 66.6 / 57.4
+//   s L TMA  7168  5.56 / 5.70 / 6.63 / 8.45    8192  7.24 / 7.21 / 8.28 / 10.4    24576 - / 111.8 / 112.1 / 117.2
+//   s U TMA  5120  3.85 / 3.90 / 4.53 / 5.98    6144  5.83 / 5.49 / 6.12 / 7.80    7168  9.00 / 7.84 / 8.07 / 10.0
+//            8192  13.4 / 11.0 / 10.6 / 12.7    12288 44.7 / 33.4 / 28.9 / 29.3    14336 70.2 / 51.6 / 43.9 / 42.5
+//   s L odd  2047  1.62 / 1.62 / 1.79 / 2.20    4001  4.38 / 3.98 / 4.10 / 4.89    5003  6.82 / 5.82 / 5.74 / 6.75
+//            10001 36.9 / 23.7 / 18.5 / 18.8    12287 67.9 / 41.4 / 29.8 / 28.2
+//   s U odd  2047  1.39 / 1.48 / 1.72 / 2.20    3001  2.47 / 2.42 / 2.79 / 3.45    6001  8.16 / 6.52 / 6.66 / 8.11
+//            7003  11.9 / 9.19 / 8.90 / 10.6    10001 35.4 / 23.8 / 19.5 / 19.7    12287 64.3 / 41.9 / 32.6 / 30.8
+//   c L      9216  33.9 / 34.1 / 35.2 / 39.6    10240 44.5 / 44.2 / 45.9 / 50.1    16384 159.6 / 154.3 / 154.2 / 160.5
+//   c U      5120  11.7 / 12.0 / 12.8 / 15.0    6144  15.9 / 15.8 / 17.7 / 20.1    10240 56.0 / 51.8 / 51.8 / 56.5
+//            24576 - / 600.6 / 586.0 / 604.6
+//   z L      4608  9.26 / 9.46 / 9.92 / 11.5    5120  11.4 / 11.0 / 12.0 / 13.7    7168  24.1 / 22.6 / 22.6 / 25.4
+//            14336 - / 140.1 / 134.2 / 134.3    20480 - / 392.3 / 373.9 / 368.5
+//   z U      4096  9.23 / 9.38 / 10.4 / 12.4    4608  12.2 / 12.0 / 13.0 / 15.5    7168  34.7 / 31.8 / 32.3 / 35.9
+//            8192  50.3 / 45.0 / 44.2 / 48.2    20480 - / 604.9 / 577.0 / 584.9
+// (odd leading dimensions of d lie at the same lines: L 6001 4.83 / 4.82, U 4001 2.87 / 2.89 for 2 / 4.)
+static int potrf_group(char type, char uplo, int n, bool tma)
 {
-    if (n < 3072) return 1;
-    if (type == 'c') return n < 6144 ? 1 : n < 12288 ? 2 : DDLAK_POTRF_GROUP;
-    return n < 6144 ? 2 : n < 12288 ? 4 : DDLAK_POTRF_GROUP;
+    constexpr int never = INT_MAX;
+    const bool up = uplo == 'U';
+    struct Lines { int two, four, eight; };
+    const Lines l = type == 'd'   ? (up ? Lines{1536, 4352, 7680} : Lines{4096, 6400, 10240})
+                    : type == 'c' ? (up ? Lines{5888, 10240, never} : Lines{9728, 16384, never})
+                    : type == 'z' ? (up ? Lines{4352, 7680, never} : Lines{4864, 7168, 14848})
+                    : tma         ? (up ? Lines{5376, 7680, 13312} : Lines{7936, never, never})
+                                  : (up ? Lines{2560, 6400, 11008} : Lines{2048, 4608, 11008});
+    return n >= l.eight ? 8 : n >= l.four ? 4 : n >= l.two ? 2 : 1;
 }
 
 template <class T>
@@ -623,5 +645,6 @@ extern "C" int ddlak_potrf_grouped(char type, char uplo, int group, int n, void*
 
 extern "C" int ddlak_potrf(char type, char uplo, int n, void* A, long long lda, int* dinfo, void* stream)
 {
-    return ddlak_potrf_grouped(type, uplo, ddlak::potrf_group(type, n), n, A, lda, dinfo, stream);
+    const bool tma = lda % 4 == 0 && (reinterpret_cast<uintptr_t>(A) & 15) == 0;  // as sg::encode for FP32
+    return ddlak_potrf_grouped(type, uplo, ddlak::potrf_group(type, uplo, n, tma), n, A, lda, dinfo, stream);
 }
