@@ -8,7 +8,8 @@
 // substitution; the backward a batched W = L^-1 and
 // the tiled (W^T W) contraction with the adjoint epilogue.  Larger orders
 // (batch 1): the blocked factorization (ddlak_potrf), the fused solve, and for
-// the backward W = L^-1 from the fused forward substitution on the identity.
+// the backward W = L^-1 (the fused forward substitution on the identity; large FP32
+// factors by doubling).
 #include <cuda_runtime.h>
 
 #include <cmath>
@@ -116,7 +117,7 @@ void factor_solve(const DdlaHandle_t& h, int batch, int n, T* A, const T* y, T* 
 }
 
 // W = L^-1 for the (W^T W) contraction: one CTA per matrix up to order 1024,
-// the fused forward substitution on the identity above.
+// ddlak_trtri_blocked above.
 template <class T>
 void inverse_factor(const DdlaHandle_t& h, int batch, int n, const T* L, T* W)
 {

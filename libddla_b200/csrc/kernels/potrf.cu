@@ -544,8 +544,8 @@ __global__ void __launch_bounds__(PB_NT) k_potrs_batched_f64(int n, const double
 
 // A batch of equal-order FP64 matrices (lower), right-looking by super-steps of
 // G block columns of 128, each step one launch per kernel over the whole batch:
-// the diagonal blocks (one CTA per matrix), the panels (row-per-thread solve,
-// grid.y = matrix) and the updates (TMA DMMA tiles, grid.y = matrix).  In a
+// the diagonal blocks (one CTA per matrix), the panels (16-row strips, grid.y = matrix;
+// both panel.cu) and the updates (TMA DMMA tiles, grid.y = matrix).  In a
 // super-step, block column g first takes the update of its own 128 columns by
 // block columns 0 .. g-1 (K = 128 g), and the rest of the trailing matrix is
 // updated once with K = 128 G, so the trailing matrix is read and written once

@@ -15,8 +15,9 @@
 // Each CTA streams the off-diagonal tiles of its block row through a
 // double-buffered cp.async ring (the tile loads do not depend on other CTAs,
 // only the solved blocks do), visiting them in publication order, then solves
-// its diagonal block with one warp per pair of right-hand sides using
-// reciprocal pivots and warp shuffles.
+// its diagonal block: the real types on the FP64 tensor cores by substitution over
+// 8 x 8 tiles (k_potrs_dmma), the complex types with one warp per pair of
+// right-hand sides using reciprocal pivots and warp shuffles (k_potrs_fused).
 //
 // The right-hand sides are a view X(i, r): B[i + r*ldb] for side 'L' and
 // conj(B[r + i*ldb]) for side 'R' (X * A = B  <=>  A * X^H = B^H, since A is

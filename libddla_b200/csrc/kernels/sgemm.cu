@@ -128,7 +128,9 @@ __global__ void __launch_bounds__(sg::NT, 2)
 }
 
 // The 64 x 64 diagonal blocks' inverses: one thread per column, four blocks per CTA, FP64
-// arithmetic, the column in registers and L through the L1 cache.
+// arithmetic, the column in registers (152 bytes of them spilled) and L through the L1 cache.
+// What bounds it: one thread's serial column, some 100 us whatever the order, which is why small
+// factors are inverted another way (kTrtriDoubling, potrs.cu).
 constexpr int SL = 64;
 __global__ void __launch_bounds__(256) k_trtri_leaf_f32(int nleaf, int n, const float* __restrict__ Lg, long long ldl,
                                                         float* __restrict__ Wg, long long ldw)

@@ -61,8 +61,8 @@ __device__ __forceinline__ void dmma2(double (&u)[2], double (&v)[2], double a_u
 //        fragments always come from lines of one parity, so the readers just add
 //        a per-lane offset.  Words past the limits are zero-filled, not read.
 // What bounds it: the DMMA pipe (FP64 tensor, 35.5 TFLOP/s by cuBLAS DGEMM); odd leading
-// dimensions cost about as much as even ones (the 16-byte copies of a slice are some 17
-// per thread against 256 DMMAs per warp).
+// dimensions take some 15 % longer (a whole factorization 57.0 ms at n = 16383, 49.6 at 16384;
+// the 16-byte copies of a slice are some 17 per thread against 256 DMMAs per warp).
 // Every wait is bounded: if one gives up, the CTA records it in g_dmma_status,
 // writes NaN into its tile (the factorization then stops at that column block with
 // a failed pivot) and waits, bounded, for its copies still in flight.
@@ -313,10 +313,12 @@ cudaError_t launch_syrk(double* A, long long lda, long long astride, int batch, 
 }  // namespace
 
 // Fewest 128 x 128 tiles for which they are used.  A region with fewer leaves SMs idle
-// (one such CTA per SM), and 64 x 64 tiles, two per SM, spread it: a whole factorization
-// at n = 2048 (look-ahead columns of 16 tiles) takes 0.86 against 1.98 ms, n = 5003 3.60
-// against 6.17 ms; at n = 16384 50.1 against 52.3 ms.  Lines at 74, 148, 296 and 592
-// tiles measured within 3 % of one another at every order.
+// (one such CTA per SM), and 64 x 64 tiles, two per SM, spread it.  ms of a whole factorization,
+// nothing else changed, with 128 x 128 tiles always / from 148 / never:
+//   lower  n = 1024 .466 / .351 / .351   2048 .974 / .756 / .750   5003 3.82 / 3.33 / 3.25
+//          8192 9.27 / 8.24 / 8.04       16384 51.6 / 49.6 / 50.5
+//   upper  2048 1.22 / .945 / .945       5003 5.09 / 4.21 / 4.13   16384 58.7 / 57.3 / 55.6
+// Lines at 74, 148 and 296 tiles are within 3 % of one another at every order.
 constexpr long long kSyrkBigTiles = 148;
 
 // The FP64 update of a batch of equal-order matrices (batch 1: one matrix, astride unused),

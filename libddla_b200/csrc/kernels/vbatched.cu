@@ -29,7 +29,7 @@
 // other's), at large ones the DMMA pipe.  Measured, time of a CTA per matrix at full
 // residency (FP64, solve included, W = 64): n = 64 30 us, 256 237 us, 512 1.04 ms; 4096
 // matrices of 16 .. 512: FP64 9.4 -> 4.4 ms, FP32 6.4 -> 4.3 ms against block columns in
-// registers on the FP64 / FP32 pipes.
+// registers on the FP64 / FP32 pipes.  At two CTAs per SM 28 (FP32) to 48 (FP64) bytes spill.
 // info follows LAPACK ?potrf (order of the first non-positive leading minor);
 // a failed matrix keeps its right-hand side and gets logdet NaN.
 #include <cuda_runtime.h>
