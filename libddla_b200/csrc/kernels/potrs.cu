@@ -328,8 +328,8 @@ __global__ void __launch_bounds__(NT) k_potrs_fused(const T* __restrict__ A, lon
 //     other three warps of its right-hand sides through shared memory.  The inverse
 //     of the whole 64 x 64 block in place of this is not backward stable: for
 //     a squared-exponential kernel on a line, condition 1e14, n = 256, the backward error
-//     was 1e-12 with 64-row inverses, 1e-15 with 16-row ones and 4e-17 with 8-row
-//     ones, as by substitution.
+//     is 1e-12 with 64-row inverses, 1e-15 with 16-row ones and 4e-17 with 8-row
+//     ones, as by substitution (restated in numpy).
 //   * One thread polls the flag of the block needed; behind it a warp looks how many of the
 //     next 32 blocks are up too, so that blocks known to be up cost no look and no fence.
 //     A block's solution goes through shared memory, four entries a thread, fetched under
