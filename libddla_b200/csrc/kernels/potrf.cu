@@ -36,8 +36,10 @@ namespace ddlak {
 // ---------------------------------------------------------------------------
 // 1. diagonal block
 // ---------------------------------------------------------------------------
+// (one CTA runs: the bound lets it use the registers.  Without, the compiler stopped at 147 for
+// single complex: 112 / 121 us for a lower / upper 128 x 128 block against 92 / 99.)
 template <class T, bool UP>
-__global__ void __launch_bounds__(256) k_potrf_diag(T* __restrict__ A, long long lda, int k0, int nbk,
+__global__ void __launch_bounds__(256, 1) k_potrf_diag(T* __restrict__ A, long long lda, int k0, int nbk,
                                                     int* __restrict__ info)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -396,9 +398,10 @@ static cudaError_t potrf_enqueue(T* A, long long lda, int n, int G, int* dinfo, 
 //            10001 36.9 / 23.7 / 18.5 / 18.8    12287 67.9 / 41.4 / 29.8 / 28.2
 //   s U odd  2047  1.39 / 1.48 / 1.72 / 2.20    3001  2.47 / 2.42 / 2.79 / 3.45    6001  8.16 / 6.52 / 6.66 / 8.11
 //            7003  11.9 / 9.19 / 8.90 / 10.6    10001 35.4 / 23.8 / 19.5 / 19.7    12287 64.3 / 41.9 / 32.6 / 30.8
-//   c L      9216  33.9 / 34.1 / 35.2 / 39.6    10240 44.5 / 44.2 / 45.9 / 50.1    16384 159.6 / 154.3 / 154.2 / 160.5
-//   c U      5120  11.7 / 12.0 / 12.8 / 15.0    6144  15.9 / 15.8 / 17.7 / 20.1    10240 56.0 / 51.8 / 51.8 / 56.5
-//            24576 - / 600.6 / 586.0 / 604.6
+//   c L      8192  24.7 / 25.1 / 26.7 / 29.8    10240 44.0 / 43.5 / 45.2 / 49.4    16384 159.1 / 153.4 / 153.6 / 159.5
+//            24576 - / 495.0 / 494.5 / 511.3
+//   c U      6144  15.5 / 15.7 / 16.7 / 19.2    7168  21.9 / 21.1 / 22.6 / 25.5    10240 55.5 / 51.0 / 51.1 / 55.3
+//            12288 91.0 / 82.6 / 80.7 / 85.7    24576 - / 600.6 / 586.0 / 604.6
 //   z L      4608  9.26 / 9.46 / 9.92 / 11.5    5120  11.4 / 11.0 / 12.0 / 13.7    7168  24.1 / 22.6 / 22.6 / 25.4
 //            14336 - / 140.1 / 134.2 / 134.3    20480 - / 392.3 / 373.9 / 368.5
 //   z U      4096  9.23 / 9.38 / 10.4 / 12.4    4608  12.2 / 12.0 / 13.0 / 15.5    7168  34.7 / 31.8 / 32.3 / 35.9
@@ -410,7 +413,7 @@ static int potrf_group(char type, char uplo, int n, bool tma)
     const bool up = uplo == 'U';
     struct Lines { int two, four, eight; };
     const Lines l = type == 'd'   ? (up ? Lines{1536, 4352, 7680} : Lines{4096, 6400, 10240})
-                    : type == 'c' ? (up ? Lines{5888, 10240, never} : Lines{9728, 16384, never})
+                    : type == 'c' ? (up ? Lines{6400, 11264, never} : Lines{9728, 16384, never})
                     : type == 'z' ? (up ? Lines{4352, 7680, never} : Lines{4864, 7168, 14848})
                     : tma         ? (up ? Lines{5376, 7680, 13312} : Lines{7936, never, never})
                                   : (up ? Lines{2560, 6400, 11008} : Lines{2048, 4608, 11008});
