@@ -334,7 +334,8 @@ int ddlak_batched_logdiag(char type, int batch, int n, const void* L, long long 
 /* Adjoint contraction on 128 x 128 lower tiles of A^-1 = W^T W (mode bit 2 set: W
  * already holds A^-1).  mode & 1 == 0: grad[m][0..2] = dloss/d{l, sigma_f^2,
  * sigma^2} through per-tile partials (partial: ddlak_adjoint_partial_bytes);
- * mode & 1 == 1: G = 1/2 (A^-1 - alpha alpha^T), dense symmetric. */
+ * mode & 1 == 1: G = 1/2 (A^-1 - alpha alpha^T), dense symmetric.  A device wait
+ * that gives up leaves NaN in its tile's results. */
 unsigned long long ddlak_adjoint_partial_bytes(int batch, int n);
 int ddlak_adjoint_contract(char type, int mode, int batch, int n, const void* W, long long ldw, long long wstride,
                            const void* alpha, long long astride, const void* X, int d, long long xstride,

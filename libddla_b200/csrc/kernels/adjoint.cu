@@ -966,6 +966,7 @@ bool contract_dmma(int mode, int batch, int n, const double* W, long long ldw, l
 
 // FP32, one matrix: the same tiles by the packed FP32 tile product (sgemm.cuh), k over
 // [i0, n); W(k, i) counts for k >= i, what lies above W's diagonal is masked.
+// The code of a wait that gave up, for a debugger: the caller sees a NaN gradient.
 __device__ int g_contract_status;
 template <int MODE, bool TMA>
 __global__ void __launch_bounds__(CT_NT, 1)

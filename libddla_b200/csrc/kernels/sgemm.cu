@@ -13,6 +13,8 @@ namespace ddlak {
 
 namespace {
 
+// The code of an update wait that gave up, for a debugger: the caller sees NaN in the tile and the
+// failed pivot it makes.
 __device__ int g_sgemm_status;
 
 // C(i, j) -= sum_{k0 <= k < k0 + nbk} L(i, k) L(j, k) on the lower tiles of the region from

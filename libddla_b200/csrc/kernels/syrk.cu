@@ -86,7 +86,7 @@ __host__ __device__ constexpr int sy_box(int rows) { return UP ? rows * sy_ld<UP
 template <class Cfg, bool UP>
 constexpr size_t sy_smem() { return (size_t)Cfg::NS * (sy_box<UP>(Cfg::BM) + sy_box<UP>(Cfg::BN)) * 8 + 128; }
 
-__device__ int g_dmma_status;
+__device__ int g_dmma_status;  // for a debugger: the caller sees the failed pivot
 
 // Where the shared copy of a line starts relative to its slice row: 1 when the line's
 // first word (A + start + line * lda) is not 16-byte aligned.
